@@ -724,17 +724,6 @@ __global__ void k_resid_grp(const ResidProb* __restrict__ probs, const uint2* __
   resid_body(P.nx, P.ny, P.nz, P.idx2, P.zop, P.rhs, P.phi, P.hi, P.lo, P.ld, int(e.y & 0xffffu), int(e.y >> 16u), int(blockIdx.z));
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// tridiagonal solves in z per mode (l, m) (solver.js:70-103): T2[k][m][l] fp32 in, S_y[k][l][m] bf16 hi/lo out.
-// Block = 32 modes in l x 16 in m; forward-sweep coefficients and the right-hand side stay in registers; the result
-// goes out through a shared-memory transpose so that every thread stores 16 consecutive m (32 bytes per output
-// row: whole sectors). The lowest 2 x 2 modes (near-singular:
-// Neumann in z, shift ~ -(pi/L)^2) use FP64 factors precomputed on the host at set_density.
-// ---------------------------------------------------------------------------------------------------------------
-// modes in m per block: 16 (whole 32-byte sectors per output row) while a thread's NZ levels fit in the 128 registers
-// of a 512-thread block, else 8
-template <int NZ>
-constexpr int tri_tm() { return NZ > 40 ? 8 : 16; }
 // the reciprocal of a mode's pivot at one level, den = diag + shift * rhoC - lower * c'_{k-1} (solver.js:88-90), with
 // c'_{k-1} in the innermost product so that nothing of it is computed ahead of the recurrence; rcp.approx is one
 // MUFU instruction, at most 1 ulp from the rounded reciprocal (the pivots are normal numbers: |den| >= the diagonal's
@@ -744,86 +733,6 @@ __device__ __forceinline__ float tri_pivot_rcp(const float4& o, float shift, flo
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
   return r;
-}
-template <int NZ>
-__device__ __forceinline__ void tri_body(int nxp, int nyp, int ldy, const float* __restrict__ lam, const float4* __restrict__ zop,
-                                         const double* __restrict__ low, const float* __restrict__ T2,
-                                         __nv_bfloat16* __restrict__ ohi, __nv_bfloat16* __restrict__ olo, const int BX, const int BY) {
-  constexpr int KC = 16;  // levels per transpose chunk
-  constexpr int TRI_TM = tri_tm<NZ>();
-  __shared__ float tile[KC][TRI_TM][33];
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + 32 * ty;
-  const int l = BX * 32 + tx, m = BY * TRI_TM + ty;
-  const bool act = l < nxp && m < nyp;
-  const bool lowm = l < 2 && m < 2;
-  const long sxy = long(nxp) * nyp;
-  float x[NZ];
-  if (act && !lowm) {
-    const float shift = __ldg(lam + l) + __ldg(lam + nxp + m);
-    const float* h = T2 + long(m) * nxp + l;
-#pragma unroll
-    for (int k = 0; k < NZ; k++) x[k] = __ldg(h + sxy * k);  // all loads issued up front; d and then x replace them
-    float cp[NZ];
-    float cprev = 0.f, dprev = 0.f;
-#pragma unroll
-    for (int k = 0; k < NZ; k++) {
-      const float4 o = __ldg(zop + k);
-      const float rd = tri_pivot_rcp(o, shift, cprev);
-      cprev = o.y * rd;
-      dprev = fmaf(-o.x, dprev, x[k]) * rd;
-      cp[k] = cprev;
-      x[k] = dprev;
-    }
-#pragma unroll
-    for (int k = NZ - 2; k >= 0; k--) x[k] = fmaf(-cp[k], x[k + 1], x[k]);
-  } else if (act) {
-    // low mode: low[(mode*2 + 0)*NZ + k] = 1/den_k, low[(mode*2 + 1)*NZ + k] = c'_k (FP64, host-factored)
-    const int mode = m * 2 + l;
-    const double* rd = low + (mode * 2) * NZ;
-    const double* cpd = rd + NZ;
-    const float* h = T2 + long(m) * nxp + l;
-    double d[NZ];
-    double dprev = 0.0;
-    for (int k = 0; k < NZ; k++) {
-      const double lo = double(__ldg(zop + k).x);
-      dprev = (double(h[sxy * k]) - lo * dprev) * rd[k];
-      d[k] = dprev;
-    }
-    for (int k = NZ - 2; k >= 0; k--) d[k] = d[k] - cpd[k] * d[k + 1];
-#pragma unroll
-    for (int k = 0; k < NZ; k++) x[k] = float(d[k]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < NZ; k++) x[k] = 0.f;
-  }
-  // transposed store, KC levels at a time: every thread then writes 8 consecutive m of one (level, l) row
-#pragma unroll
-  for (int kc = 0; kc < NZ; kc += KC) {
-#pragma unroll
-    for (int kk = 0; kk < KC; kk++)
-      if (kc + kk < NZ) tile[kk][ty][tx] = x[kc + kk];
-    __syncthreads();
-    const int nkc = NZ - kc < KC ? NZ - kc : KC;
-    for (int t = tid; t < nkc * 32; t += 32 * TRI_TM) {
-      const int kk = t >> 5, lx = t & 31;
-      const int ll = BX * 32 + lx;
-      if (ll < nxp) {
-        __align__(16) __nv_bfloat16 h16[TRI_TM], l16[TRI_TM];
-#pragma unroll
-        for (int u = 0; u < TRI_TM; u++) tc::split_bf16(tile[kk][u][lx], h16[u], l16[u]);
-        // rows hold ldy (a multiple of 8) values: 16-byte aligned; columns past nyp land in the row's zero padding
-        // when the pitch has room for them, else they are skipped
-        const long o = (long(kc + kk) * nxp + ll) * ldy + BY * TRI_TM;
-#pragma unroll
-        for (int h = 0; h < TRI_TM / 8; h++)
-          if (BY * TRI_TM + h * 8 + 8 <= ldy) {
-            *reinterpret_cast<uint4*>(ohi + o + h * 8) = *reinterpret_cast<const uint4*>(h16 + h * 8);
-            if (olo) *reinterpret_cast<uint4*>(olo + o + h * 8) = *reinterpret_cast<const uint4*>(l16 + h * 8);
-          }
-      }
-    }
-    __syncthreads();
-  }
 }
 // ---------------------------------------------------------------------------------------------------------------
 // The tridiagonals of one model's solve through shared memory, every transfer a TMA tile (solver.js:70-103).
@@ -841,6 +750,8 @@ __device__ __forceinline__ void tri_body(int nxp, int nyp, int ldy, const float*
 //      doubled the L2 write transactions and made L2 fetch sectors back from DRAM).
 // 64 registers and NZ KB of shared memory per 256-thread block (NZ <= 40: four blocks per SM), so one block's loads
 // overlap another's sweeps and stores.
+// T2's rows are padded to whole 16 bytes, so that every width has its tensor maps: at 333 x 275 x 40 a launch takes
+// 18.9 us under ncu against 20.1 us for the kernel with plain loads and stores that rows of other lengths needed before.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int TRI_TL = 16, TRI_TM = 16;
 template <int NZ>
@@ -1023,45 +934,6 @@ __global__ void __launch_bounds__(TRI_TL * TRI_TM, NZ > 40 ? 2 : 4) k_tri_tma_gr
   tri_tma_tile<NZ, HI_ONLY>(&P->in, &P->hi, &P->lo, P->nxp, P->nyp, P->lam, [&](int k) { return zs[k]; }, P->low, err,
                             (r % gx) * TRI_TL, (r / gx) * TRI_TM, smraw);
 }
-// the same solve with plain loads and stores (tri_body), for planes whose pitch a tensor map cannot describe (T2's
-// row pitch nxp * 4 bytes not a multiple of 16)
-template <int NZ>
-__global__ void __launch_bounds__(32 * tri_tm<NZ>()) k_tri_tc(int nxp, int nyp, int ldy, const float* __restrict__ lam, const float4* __restrict__ zop,
-                                                const double* __restrict__ low, const float* __restrict__ T2,
-                                                __nv_bfloat16* __restrict__ ohi, __nv_bfloat16* __restrict__ olo) {
-  tri_body<NZ>(nxp, nyp, ldy, lam, zop, low, T2, ohi, olo, blockIdx.x, blockIdx.y);
-}
-// the tridiagonals of every member of an ensemble: member p owns the linear blocks [start[p], start[p+1])
-struct TriProb {
-  int nxp, nyp, ldy, gx;
-  const float* lam;
-  const float4* zop;
-  const double* low;
-  const float* T2;
-  __nv_bfloat16* ohi;
-  __nv_bfloat16* olo;
-};
-template <int NZ>
-__global__ void __launch_bounds__(32 * tri_tm<NZ>()) k_tri_tc_grp(const TriProb* __restrict__ probs, const int* __restrict__ start, int n) {
-  // one thread finds the block's member; the problem is read from shared memory, so that no register holds it
-  // through the sweeps
-  __shared__ TriProb P;
-  __shared__ int r;
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    const int b = blockIdx.x;
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(start + mid) <= b) lo = mid;
-      else hi = mid - 1;
-    }
-    P = probs[lo];
-    r = b - __ldg(start + lo);
-  }
-  __syncthreads();
-  tri_body<NZ>(P.nxp, P.nyp, P.ldy, P.lam, P.zop, P.low, P.T2, P.ohi, P.olo, r % P.gx, r / P.gx);
-}
-
 // ---------------------------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------------------------
@@ -1150,18 +1022,13 @@ static void set_smem_attrs() {
     cudaFuncSetAttribute(k_dst_tc2<OUT_T_F32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
     cudaFuncSetAttribute(k_dst_tc2<OUT_R_F32_ADD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
     cudaFuncSetAttribute(k_dst_tc2<OUT_R_F32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
-    cudaFuncSetAttribute(k_tri_tma<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<16>());
-    cudaFuncSetAttribute(k_tri_tma<40, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<40>());
-    cudaFuncSetAttribute(k_tri_tma<80, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<80>());
-    cudaFuncSetAttribute(k_tri_tma<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<16>());
-    cudaFuncSetAttribute(k_tri_tma_grp<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<16>());
-    cudaFuncSetAttribute(k_tri_tma_grp<40, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<40>());
-    cudaFuncSetAttribute(k_tri_tma_grp<80, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<80>());
-    cudaFuncSetAttribute(k_tri_tma_grp<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<16>());
-    cudaFuncSetAttribute(k_tri_tma_grp<40, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<40>());
-    cudaFuncSetAttribute(k_tri_tma_grp<80, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<80>());
-    cudaFuncSetAttribute(k_tri_tma<40, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<40>());
-    cudaFuncSetAttribute(k_tri_tma<80, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<80>());
+#define OB_ATTR(NZ)                                                                                                            \
+    cudaFuncSetAttribute(k_tri_tma<NZ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<NZ>());     \
+    cudaFuncSetAttribute(k_tri_tma<NZ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<NZ>());      \
+    cudaFuncSetAttribute(k_tri_tma_grp<NZ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<NZ>()); \
+    cudaFuncSetAttribute(k_tri_tma_grp<NZ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri_smem_bytes<NZ>());
+    OB_ATTR(16) OB_ATTR(40) OB_ATTR(80)
+#undef OB_ATTR
     attr = true;
   }
 }
@@ -1187,7 +1054,7 @@ struct TcPlan {
   int qdim[4] = {};
   CUtensorMap Fx[2], Fy[2], Fr[2], Frr[2];  // fields, the A operand: S_x, S_y, the split right-hand side and residual
   CUtensorMap tri_in, tri_out[2];  // the tridiagonals' tiles: T2[k][m][l] fp32 in, S_y[k][l][m] bf16 hi / lo out
-  bool tri_tma = false;
+  long ld2 = 0;          // row pitch of T2 (floats, whole 16 bytes: the tensor map's rule)
   float4 zh[80] = {};    // the z-operator on the host: the by-value coefficients of k_tri_tma (nz <= 80)
   CUtensorMap Qh[4][2];  // the DST matrices with boxes of half a tile's width: each CTA of a pair loads one half
   bool pairs = true;     // transforms on SM pairs (k_dst_tc2); single-SM tiles (k_dst_tc) when false
@@ -1231,12 +1098,13 @@ int PoissonPlan::tc_create() {
   T->nx = nx; T->ny = ny; T->nz = nz;
   T->ldx = pad8(nx);
   T->ldy = pad8(ny);
+  T->ld2 = (nx + 3) / 4 * 4;
   const size_t mx = size_t(nx) * T->ldx, my = size_t(ny) * T->ldy;
   const size_t nsx = size_t(nz) * ny * T->ldx, nsy = size_t(nz) * nx * T->ldy;
   auto al = [&](void** p, size_t bytes) { return cudaMalloc(p, bytes) == cudaSuccess && cudaMemset(*p, 0, bytes) == cudaSuccess; };
   bool ok = al((void**)&T->mat, (4 * mx + 4 * my) * 2) && al((void**)&T->sx_hi, nsx * 2) && al((void**)&T->sx_lo, nsx * 2) &&
             al((void**)&T->rx_hi, nsx * 2) && al((void**)&T->rx_lo, nsx * 2) &&
-            al((void**)&T->sy_hi, nsy * 2) && al((void**)&T->sy_lo, nsy * 2) && al((void**)&T->t2, size_t(nz) * nx * ny * 4) &&
+            al((void**)&T->sy_hi, nsy * 2) && al((void**)&T->sy_lo, nsy * 2) && al((void**)&T->t2, size_t(nz) * T->ld2 * ny * 4) &&
             al((void**)&T->low, size_t(8) * nz * 8) && al((void**)&T->err, 16);
   if (ok && precision >= 2) ok = al((void**)&T->rr_hi, nsx * 2) && al((void**)&T->rr_lo, nsx * 2);
   if (!ok) {
@@ -1277,15 +1145,17 @@ int PoissonPlan::tc_create() {
     set_error("poisson: tensor map encoding failed");
     return OB_ERR_DEVICE;
   }
-  // the tridiagonals' tiles (k_tri_tma); when T2's row pitch is not a multiple of 16 bytes the plain-load kernel runs
-  if ((nz == 16 || nz == 40 || nz == 80) && (long(nx) * 4) % 16 == 0) {
-    const long din[3] = {nx, ny, nz}, pin[2] = {long(nx) * 4, long(nx) * ny * 4};
-    const int bin[3] = {TRI_TL, TRI_TM, nz};
-    const long dout[3] = {T->ldy, nx, nz}, pout[2] = {T->ldy * 2, T->ldy * nx * 2};
-    const int bout[3] = {TRI_TM, TRI_TL, nz};
-    T->tri_tma = make_map_3d(&T->tri_in, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, T->t2, din, pin, bin) &&
-                 make_map_3d(&T->tri_out[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, T->sy_hi, dout, pout, bout) &&
-                 make_map_3d(&T->tri_out[1], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, T->sy_lo, dout, pout, bout);
+  // the tridiagonals' tiles (k_tri_tma); a plan of other level counts has none (tc_solve refuses it)
+  const bool tri = nz == 16 || nz == 40 || nz == 80;
+  const long din[3] = {nx, ny, nz}, pin[2] = {T->ld2 * 4, T->ld2 * ny * 4};
+  const int bin[3] = {TRI_TL, TRI_TM, nz};
+  const long dout[3] = {T->ldy, nx, nz}, pout[2] = {T->ldy * 2, T->ldy * nx * 2};
+  const int bout[3] = {TRI_TM, TRI_TL, nz};
+  if (tri && !(make_map_3d(&T->tri_in, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, T->t2, din, pin, bin) &&
+               make_map_3d(&T->tri_out[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, T->sy_hi, dout, pout, bout) &&
+               make_map_3d(&T->tri_out[1], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, T->sy_lo, dout, pout, bout))) {
+    set_error("poisson: tensor map encoding failed");
+    return OB_ERR_DEVICE;
   }
   set_smem_attrs();
   pair_slots();   // the occupancy query of the paired transform runs here, outside any stream capture
@@ -1419,11 +1289,11 @@ static void launch_tri_tma(const TcPlan* T, const float* lam, bool hi_only, cuda
 
 // the four transforms and the tridiagonals from a split right-hand side (rx, or the residual rr when add) to phi
 // (stored, or added when add)
-static void tc_pass(const PoissonPlan& P, TcPlan* T, const float* lam, const float4* zop, float* phi, bool add, cudaStream_t s,
+static void tc_pass(const PoissonPlan& P, TcPlan* T, const float* lam, float* phi, bool add, cudaStream_t s,
                     bool one = false) {
 #define QH(t) (T->pairs ? T->Qh[t] : nullptr)
   const int nx = P.nx, ny = P.ny, nz = P.nz;
-  const TcOut sy{T->sy_hi, T->sy_lo, nullptr, T->ldy, ny, nz * ny, nx}, t2{nullptr, nullptr, T->t2, nx, nx, nz * nx, ny};
+  const TcOut sy{T->sy_hi, T->sy_lo, nullptr, T->ldy, ny, nz * ny, nx}, t2{nullptr, nullptr, T->t2, T->ld2, nx, nz * nx, ny};
   // X-fwd: field rows (k, j), K = i, outputs l  -> S_y[k][l][j]
   if (one) launch_tc<OUT_T_BF16X2, true>(add ? T->Frr : T->Fr, T->Q[0], nx, T->bnx, sy, T->err, s, QH(0));
   else launch_tc<OUT_T_BF16X2>(add ? T->Frr : T->Fr, T->Q[0], nx, T->bnx, sy, T->err, s, QH(0));
@@ -1432,19 +1302,10 @@ static void tc_pass(const PoissonPlan& P, TcPlan* T, const float* lam, const flo
   else launch_tc<OUT_T_F32>(T->Fy, T->Q[1], ny, T->bny, t2, T->err, s, QH(1));
   // tridiagonals -> S_y[k][l][m]
   // (a plain-bf16 pass writes the hi plane alone: its y-inverse transform reads nothing else)
-  if (T->tri_tma) {
-    switch (nz) {
-      case 16: launch_tri_tma<16>(T, lam, one, s); break;
-      case 40: launch_tri_tma<40>(T, lam, one, s); break;
-      default: launch_tri_tma<80>(T, lam, one, s); break;
-    }
-  } else {
-    __nv_bfloat16* lo = one ? nullptr : T->sy_lo;
-    switch (nz) {
-      case 16: k_tri_tc<16><<<dim3((nx + 31) / 32, (ny + tri_tm<16>() - 1) / tri_tm<16>()), dim3(32, tri_tm<16>()), 0, s>>>(nx, ny, int(T->ldy), lam, zop, T->low, T->t2, T->sy_hi, lo); break;
-      case 40: k_tri_tc<40><<<dim3((nx + 31) / 32, (ny + tri_tm<40>() - 1) / tri_tm<40>()), dim3(32, tri_tm<40>()), 0, s>>>(nx, ny, int(T->ldy), lam, zop, T->low, T->t2, T->sy_hi, lo); break;
-      default: k_tri_tc<80><<<dim3((nx + 31) / 32, (ny + tri_tm<80>() - 1) / tri_tm<80>()), dim3(32, tri_tm<80>()), 0, s>>>(nx, ny, int(T->ldy), lam, zop, T->low, T->t2, T->sy_hi, lo); break;
-    }
+  switch (nz) {
+    case 16: launch_tri_tma<16>(T, lam, one, s); break;
+    case 40: launch_tri_tma<40>(T, lam, one, s); break;
+    default: launch_tri_tma<80>(T, lam, one, s); break;
   }
   // Y-inv: field rows (k, l), K = m, outputs j  -> S_x[k][j][l]
   const TcOut sx{T->sx_hi, T->sx_lo, nullptr, T->ldx, nx, nz * nx, ny};
@@ -1473,12 +1334,12 @@ int PoissonPlan::tc_solve(const float* rhs, float* phi, cudaStream_t s) {
     if (!rhs) { set_error("poisson: right-hand side missing"); return OB_ERR_INVALID; }
   }
   if (!presplit) k_split_rows<<<1184, 256, 0, s>>>(rhs, long(nz) * ny, nx, T->rx_hi, T->rx_lo, int(T->ldx));
-  tc_pass(*this, T, lam, zop, phi, false, s, precision == 5);
+  tc_pass(*this, T, lam, phi, false, s, precision == 5);
   if (precision >= 2) {
     const int sweeps = precision == 4 ? 2 : 1;
     for (int sw = 0; sw < sweeps; sw++) {
       k_resid<<<dim3((nx + 127) / 128, ny, nz), 128, 0, s>>>(nx, ny, nz, 1.0 / (dx * dx), zop, rhs, phi, T->rr_hi, T->rr_lo, int(T->ldx));
-      tc_pass(*this, T, lam, zop, phi, true, s, precision == 3);
+      tc_pass(*this, T, lam, phi, true, s, precision == 3);
     }
   }
   const cudaError_t e = cudaGetLastError();
@@ -1546,10 +1407,7 @@ struct TcGroup {
   std::vector<const float*> rhs;
   GemmProb* d_probs = nullptr;  // [5][n]: x-fwd, y-fwd, y-inv, x-inv, x-fwd of the residual
   int* d_start = nullptr;       // [5][n + 1] tile starts, [n + 1] tridiagonal block starts, [n + 1] residual block starts
-  TriProb* d_tri = nullptr;
-  TriTmaProb* d_tri_tma = nullptr;  // the TMA tridiagonals' per-member maps, when every member has them
-  bool tri_tma = false;
-  int tri_tma_blocks = 0;
+  TriTmaProb* d_tri_tma = nullptr;  // the tridiagonals' per-member maps
   ResidProb* d_res = nullptr;
   uint2* d_res_map = nullptr;  // block map of the residual launch
   unsigned int* err = nullptr;
@@ -1562,13 +1420,10 @@ static int tc_group_build(TcGroup* G) {
   const int n = G->n;
   constexpr int NT = 5;  // transform lists
   std::vector<GemmProb> probs(size_t(NT) * n);
-  std::vector<int> start(size_t(NT + 3) * (n + 1), 0);
+  std::vector<int> start(size_t(NT + 2) * (n + 1), 0);
   std::vector<TriTmaProb> trit(n);
-  bool all_tma = true;
-  std::vector<TriProb> tri(n);
   std::vector<ResidProb> res(n);
   std::vector<uint2> res_map;
-  const int tm = G->nz == 16 ? tri_tm<16>() : G->nz == 40 ? tri_tm<40>() : tri_tm<80>();
   for (int i = 0; i < n; i++) {
     const PoissonPlan* P = G->plans[i];
     TcPlan* T = static_cast<TcPlan*>(P->tc);
@@ -1578,7 +1433,7 @@ static int tc_group_build(TcGroup* G) {
     const int bn[NT] = {bnx, bny, bny, bnx, bnx}, K[NT] = {nx, ny, ny, nx, nx}, qi[NT] = {0, 1, 2, 3, 0};
     const CUtensorMap* F[NT] = {T->Fr, T->Fy, T->Fy, T->Fx, G->precision >= 2 ? T->Frr : T->Fr};
     const TcOut xfwd{T->sy_hi, T->sy_lo, nullptr, T->ldy, ny, nz * ny, nx};
-    const TcOut out[NT] = {xfwd, TcOut{nullptr, nullptr, T->t2, nx, nx, nz * nx, ny}, TcOut{T->sx_hi, T->sx_lo, nullptr, T->ldx, nx, nz * nx, ny},
+    const TcOut out[NT] = {xfwd, TcOut{nullptr, nullptr, T->t2, T->ld2, nx, nz * nx, ny}, TcOut{T->sx_hi, T->sx_lo, nullptr, T->ldx, nx, nz * nx, ny},
                            TcOut{nullptr, nullptr, G->phi[i], nx, ny, nz * ny, nx}, xfwd};
     for (int t = 0; t < NT; t++) {
       GemmProb& g = probs[size_t(t) * n + i];
@@ -1597,27 +1452,20 @@ static int tc_group_build(TcGroup* G) {
       const int nt = ((out[t].M + BM - 1) / BM) * g.ntn;
       start[size_t(t) * (n + 1) + i + 1] = start[size_t(t) * (n + 1) + i] + nt;
     }
-    {  // the TMA tiles of 16 x 16 modes (k_tri_tma_grp), when this member's plan has their maps
-      const int tx16 = (nx + TRI_TL - 1) / TRI_TL, ty16 = (ny + TRI_TM - 1) / TRI_TM;
-      all_tma = all_tma && T->tri_tma;
-      TriTmaProb& q = trit[i];
-      std::memset(&q, 0, sizeof(q));
-      if (T->tri_tma) {
-        q.in = T->tri_in;
-        q.hi = T->tri_out[0];
-        q.lo = T->tri_out[1];
-      }
-      q.lam = P->lam;
-      q.zop = P->zop;
-      q.low = T->low;
-      q.nxp = nx;
-      q.nyp = ny;
-      q.gx = tx16;
-      start[size_t(NT + 2) * (n + 1) + i + 1] = start[size_t(NT + 2) * (n + 1) + i] + tx16 * ty16;
-    }
-    const int gx = (nx + 31) / 32, gy = (ny + tm - 1) / tm;
-    tri[i] = TriProb{nx, ny, int(T->ldy), gx, P->lam, P->zop, T->low, T->t2, T->sy_hi, T->sy_lo};
-    start[size_t(NT) * (n + 1) + i + 1] = start[size_t(NT) * (n + 1) + i] + gx * gy;
+    // the tridiagonals' tiles of 16 x 16 modes (k_tri_tma_grp)
+    const int tx16 = (nx + TRI_TL - 1) / TRI_TL, ty16 = (ny + TRI_TM - 1) / TRI_TM;
+    TriTmaProb& q = trit[i];
+    std::memset(&q, 0, sizeof(q));
+    q.in = T->tri_in;
+    q.hi = T->tri_out[0];
+    q.lo = T->tri_out[1];
+    q.lam = P->lam;
+    q.zop = P->zop;
+    q.low = T->low;
+    q.nxp = nx;
+    q.nyp = ny;
+    q.gx = tx16;
+    start[size_t(NT) * (n + 1) + i + 1] = start[size_t(NT) * (n + 1) + i] + tx16 * ty16;
     const int rgx = (nx + 127) / 128;
     res[i] = ResidProb{nx, ny, nz, int(T->ldx), 1.0 / (P->dx * P->dx), P->zop, G->rhs[i], G->phi[i], T->rr_hi, T->rr_lo};
     for (int by = 0; by < ny; by++)
@@ -1627,11 +1475,8 @@ static int tc_group_build(TcGroup* G) {
   for (int t = 0; t < NT; t++) G->tiles[t] = start[size_t(t) * (n + 1) + n];
   G->tri_blocks = start[size_t(NT) * (n + 1) + n];
   G->res_blocks = start[size_t(NT + 1) * (n + 1) + n];
-  G->tri_tma = all_tma;
-  G->tri_tma_blocks = start[size_t(NT + 2) * (n + 1) + n];
   const bool ok = cudaMemcpy(G->d_probs, probs.data(), probs.size() * sizeof(GemmProb), cudaMemcpyHostToDevice) == cudaSuccess &&
                   cudaMemcpy(G->d_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-                  cudaMemcpy(G->d_tri, tri.data(), tri.size() * sizeof(TriProb), cudaMemcpyHostToDevice) == cudaSuccess &&
                   cudaMemcpy(G->d_tri_tma, trit.data(), trit.size() * sizeof(TriTmaProb), cudaMemcpyHostToDevice) == cudaSuccess &&
                   cudaMemcpy(G->d_res, res.data(), res.size() * sizeof(ResidProb), cudaMemcpyHostToDevice) == cudaSuccess &&
                   cudaMemcpy(G->d_res_map, res_map.data(), res_map.size() * sizeof(uint2), cudaMemcpyHostToDevice) == cudaSuccess;
@@ -1644,7 +1489,7 @@ static int tc_group_build(TcGroup* G) {
 
 void tc_group_destroy(TcGroup* G) {
   if (!G) return;
-  for (void* p : {(void*)G->d_probs, (void*)G->d_start, (void*)G->d_tri, (void*)G->d_tri_tma, (void*)G->d_res, (void*)G->d_res_map, (void*)G->err})
+  for (void* p : {(void*)G->d_probs, (void*)G->d_start, (void*)G->d_tri_tma, (void*)G->d_res, (void*)G->d_res_map, (void*)G->err})
     if (p) cudaFree(p);
   delete G;
 }
@@ -1689,8 +1534,7 @@ int tc_group_create(PoissonPlan* const* plans, float* const* phi, const float* c
     return OB_ERR_INVALID;
   }
   const bool ok = cudaMalloc(&G->d_probs, size_t(5) * n * sizeof(GemmProb)) == cudaSuccess &&
-                  cudaMalloc(&G->d_start, size_t(8) * (n + 1) * sizeof(int)) == cudaSuccess &&
-                  cudaMalloc(&G->d_tri, size_t(n) * sizeof(TriProb)) == cudaSuccess &&
+                  cudaMalloc(&G->d_start, size_t(7) * (n + 1) * sizeof(int)) == cudaSuccess &&
                   cudaMalloc(&G->d_tri_tma, size_t(n) * sizeof(TriTmaProb)) == cudaSuccess &&
                   cudaMalloc(&G->d_res, size_t(n) * sizeof(ResidProb)) == cudaSuccess && cudaMalloc(&G->err, 16) == cudaSuccess &&
                   cudaMalloc(&G->d_res_map, res_map_blocks(plans, n) * sizeof(uint2)) == cudaSuccess &&
@@ -1738,23 +1582,16 @@ static void tc_group_pass(const TcGroup* G, bool add, cudaStream_t s, bool one =
     launch_tc_grp<OUT_T_F32>(G, 1, s);
   }
   const int* ts = G->d_start + size_t(5) * (n + 1);
-  if (G->tri_tma) {   // TMA tiles; a plain-bf16 pass writes the hi plane alone
-    const int* tt = G->d_start + size_t(7) * (n + 1);
-    const int nb = G->tri_tma_blocks, th = TRI_TL * TRI_TM;
-#define OB_TRI_GRP(NZ)                                                                                        \
-    if (one) k_tri_tma_grp<NZ, true><<<nb, th, tri_smem_bytes<NZ>(), s>>>(G->d_tri_tma, tt, n, G->err);      \
-    else k_tri_tma_grp<NZ, false><<<nb, th, tri_smem_bytes<NZ>(), s>>>(G->d_tri_tma, tt, n, G->err);
-    switch (G->nz) {
-      case 16: OB_TRI_GRP(16) break;
-      case 40: OB_TRI_GRP(40) break;
-      default: OB_TRI_GRP(80) break;
-    }
-#undef OB_TRI_GRP
-  } else switch (G->nz) {
-    case 16: k_tri_tc_grp<16><<<G->tri_blocks, dim3(32, tri_tm<16>()), 0, s>>>(G->d_tri, ts, n); break;
-    case 40: k_tri_tc_grp<40><<<G->tri_blocks, dim3(32, tri_tm<40>()), 0, s>>>(G->d_tri, ts, n); break;
-    default: k_tri_tc_grp<80><<<G->tri_blocks, dim3(32, tri_tm<80>()), 0, s>>>(G->d_tri, ts, n); break;
+  const int nb = G->tri_blocks, th = TRI_TL * TRI_TM;   // a plain-bf16 pass writes the hi plane alone
+#define OB_TRI_GRP(NZ)                                                                                    \
+  if (one) k_tri_tma_grp<NZ, true><<<nb, th, tri_smem_bytes<NZ>(), s>>>(G->d_tri_tma, ts, n, G->err);    \
+  else k_tri_tma_grp<NZ, false><<<nb, th, tri_smem_bytes<NZ>(), s>>>(G->d_tri_tma, ts, n, G->err);
+  switch (G->nz) {
+    case 16: OB_TRI_GRP(16) break;
+    case 40: OB_TRI_GRP(40) break;
+    default: OB_TRI_GRP(80) break;
   }
+#undef OB_TRI_GRP
   if (one) {
     launch_tc_grp<OUT_T_BF16X2, true>(G, 2, s);
     if (add) launch_tc_grp<OUT_R_F32_ADD, true>(G, 3, s);
