@@ -3,13 +3,14 @@
 //   rho_c(z) lap_h(phi) + d/dz(rho_w(z) d phi/dz) = rhs,  phi = 0 beyond the lateral faces, Neumann at ground / lid.
 //
 // Orthonormal DST-II in x and y (four dense transforms), one tridiagonal per horizontal mode (l, m) in z.
-//   precision 0: fp32 SIMT transforms (tiled GEMM, 64 x 64 tiles, fp32 FMA) — the reference's own precision;
+//   precision 0: fp32 SIMT transforms (tiled GEMM, fp32 FMA) — the reference's own precision;
 //   precision 1: bf16x3 tensor-core transforms (ob_dst_tc.cu) with fp32 accumulation; 2: plus a bf16x3
 //   refinement sweep on the FP64-accumulated residual; 3: that sweep in plain bf16.
-// The tridiagonals: fp32 Thomas with the forward-sweep coefficients in registers for every mode except the lowest
+// The tridiagonals: fp32 Thomas with the column in shared memory for every mode except the lowest
 // 2 x 2 modes, which are near-singular (Neumann in z, shift ~ -(pi/L)^2) and run in FP64.
 #include <cstdio>
 #include <cmath>
+#include <cstdint>
 #include <vector>
 
 #include "ob_poisson.cuh"
@@ -17,54 +18,144 @@
 namespace ob {
 
 // ---------------------------------------------------------------------------------------------------------------
-// fp32 SIMT batched GEMM: C(r, c) = sum_q A(r, q) B(q, c), C column-major (ldc), generic strides for A and B
+// fp32 transforms as SIMT GEMMs: C(r, c) = sum_q R(r, q) B(q, c), one fmaf chain per output with q ascending, so no
+// tile shape or split changes a bit of the result.
+//
+// What bounds it is the fp32 pipe next to shared-memory reads, which deliver 128 bytes per clock and SM whether or not
+// lanes share an address: a thread that owns r x c outputs reads 4 (r + c) bytes per r c FMAs. 8 x 8 outputs per thread
+// would need all of it, 16 x 4 more (measured: shared memory 86 % busy, 390 us per transform at 464 x 464 x 60), 16 x 8
+// needs three quarters: 288 us there (under ncu; the fp32 pipe 67-74 % busy, shared memory 60 %), against 546 us for
+// 64 x 64 tiles with 4 x 4 outputs per thread; a whole solve 2.08 -> 1.06 ms. The rows a thread owns are read as float4,
+// which are the register pairs of the packed fma.rn.f32x2 (two fmaf in one instruction, each rounded as fmaf is, and
+// half the issue slots), the columns as float2. Tiles: BR = 32 GR rows (the output's contiguous dimension) x BC = 16 CPT
+// columns by 4 warps that share all the rows and own 4 CPT columns each; the side that spans the DST matrix is 96 or
+// 128 wide, whichever pads its extent less (656 = 6.8 x 96, but 5.1 x 128). A ring of GST stages of GBK q-values is
+// filled by 4-byte cp.async (zero beyond the edges), which transposes into [q][row] on the way and asks nothing of the
+// alignment of the caller's pointers or of odd row lengths.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int GBM = 64, GBN = 64, GBK = 16;
-__global__ void __launch_bounds__(256) k_gemm_f32(int M, int N, int K, const float* __restrict__ A, long sar, long saq,
-                                                  const float* __restrict__ B, long sbq, long sbc, float* __restrict__ C,
-                                                  long ldc, long bA, long bB, long bC) {
-  __shared__ float As[GBK][GBM + 4];
-  __shared__ float Bs[GBK][GBN + 4];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int r0 = blockIdx.x * GBM, c0 = blockIdx.y * GBN;
-  A += bA * blockIdx.z;
-  B += bB * blockIdx.z;
-  C += bC * blockIdx.z;
-  float acc[4][4] = {};
-  for (int q0 = 0; q0 < K; q0 += GBK) {
+constexpr int GBK = 16, GST = 4, GTH = 128;
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool in) {
+  const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+// acc.{x,y} += a.{x,y} * b, each as fmaf
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+template <int GR, int CPT>
+constexpr int gemm_smem_bytes() { return GST * GBK * (32 * GR + 4 + 16 * CPT + 4) * 4; }
+
+// XT: x-transform. Rows = outputs l of the matrix Mx[l][q], columns = field rows (j, k): B(q, c) = src[q + K c],
+//     C[l + nx c].
+// otherwise y-transform. Rows = (k, i) of the field: R(r, q) = src[i + nx q + pl k]; columns = outputs m of the matrix
+//     My[m][q], C[i + nx m + pl k].
+template <bool XT, int GR, int CPT>
+__global__ void __launch_bounds__(GTH, 2) k_gemm_f32(int M, int N, int K, const float* __restrict__ mat, const float* __restrict__ src,
+                                                     float* __restrict__ C, int nx, long pl, int mtiles) {
+  static_assert(XT || GR == 4, "the y-transform loads one field row per thread");
+  constexpr int BR = 32 * GR, BC = 16 * CPT, LR = BR + 4, LC = BC + 4, STG = GBK * (LR + LC);
+  extern __shared__ __align__(16) float sm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lx = lane & 7, ly = lane >> 3;
+  // the matrix's tiles vary fastest, so that blocks running together share a field tile through L2
+  const int bm = int(blockIdx.x % unsigned(mtiles)), bf = int(blockIdx.x / unsigned(mtiles));
+  const int r0 = (XT ? bm : bf) * BR, c0 = (XT ? bf : bm) * BC;
+  // this thread's cp.async lines: K-contiguous operands take (q = tid & 15, 8 lines per pass); the y-transform's field
+  // rows take row tid, one q-value per pass
+  const int kq = tid & 15, kl = tid >> 4;
+  const float* rbase;   // rows operand
+  bool rin = true;
+  if (XT) {
+    rbase = mat + long(r0 + kl) * K + kq;
+  } else {
+    const int r = r0 + tid;
+    rin = r < M;
+    const int k = r / nx, i = r - k * nx;
+    rbase = src + (rin ? long(k) * pl + i : 0);
+  }
+  const float* cbase = (XT ? src : mat) + long(c0 + kl) * K + kq;
+  auto load = [&](int kt) {
+    float* s = sm + (kt % GST) * STG;
+    const int q0 = kt * GBK;
+    const bool qin = q0 + kq < K;
+    if (XT) {
 #pragma unroll
-    for (int s = 0; s < 4; s++) {
-      const int e = tid + 256 * s;
-      int r, q;
-      if (saq == 1) { q = e % GBK; r = e / GBK; } else { r = e % GBM; q = e / GBM; }
-      const int gr = r0 + r, gq = q0 + q;
-      As[q][r] = (gr < M && gq < K) ? __ldg(A + gr * sar + gq * saq) : 0.f;
-      int c, qb;
-      if (sbq == 1) { qb = e % GBK; c = e / GBK; } else { c = e % GBN; qb = e / GBN; }
-      const int gc = c0 + c, gqb = q0 + qb;
-      Bs[qb][c] = (gc < N && gqb < K) ? __ldg(B + gqb * sbq + gc * sbc) : 0.f;
+      for (int p = 0; p < BR / 8; p++) {
+        const bool in = r0 + kl + 8 * p < M && qin;
+        cp_async4(s + kq * LR + kl + 8 * p, in ? rbase + long(8 * p) * K + q0 : mat, in);
+      }
+    } else {
+#pragma unroll
+      for (int p = 0; p < GBK; p++) {
+        const bool in = rin && q0 + p < K;
+        cp_async4(s + p * LR + tid, in ? rbase + long(q0 + p) * nx : src, in);
+      }
     }
-    __syncthreads();
+    float* sc = s + GBK * LR;
+#pragma unroll
+    for (int p = 0; p < BC / 8; p++) {
+      const bool in = c0 + kl + 8 * p < N && qin;
+      cp_async4(sc + kq * LC + kl + 8 * p, in ? cbase + long(8 * p) * K + q0 : mat, in);
+    }
+  };
+  uint64_t acc[2 * GR][CPT];
+#pragma unroll
+  for (int a = 0; a < 2 * GR; a++)
+#pragma unroll
+    for (int c = 0; c < CPT; c++) acc[a][c] = 0ull;
+  const int nk = (K + GBK - 1) / GBK;
+#pragma unroll
+  for (int t = 0; t < GST - 1; t++) {
+    if (t < nk) load(t);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int kt = 0; kt < nk; kt++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(GST - 2) : "memory");
+    __syncthreads();   // stage kt has arrived for every thread, and every thread is done with the stage refilled below
+    if (kt + GST - 1 < nk) load(kt + GST - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* s = sm + (kt % GST) * STG;
+    const float* rs = s + lx * 4;
+    const float* cs = s + GBK * LR + warp * 4 * CPT + ly * 2;   // columns 8 h + 2 ly + {0, 1} of the warp's
 #pragma unroll
     for (int kk = 0; kk < GBK; kk++) {
-      float a[4], b[4];
+      ulonglong2 a[GR];
 #pragma unroll
-      for (int t = 0; t < 4; t++) { a[t] = As[kk][tx + 16 * t]; b[t] = Bs[kk][ty + 16 * t]; }
+      for (int g = 0; g < GR; g++) a[g] = *reinterpret_cast<const ulonglong2*>(rs + kk * LR + 32 * g);
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int h = 0; h < CPT / 2; h++) {
+        const float2 b = *reinterpret_cast<const float2*>(cs + kk * LC + 8 * h);
+        uint64_t bx, by;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(bx) : "f"(b.x));
+        asm("mov.b64 %0, {%1, %1};" : "=l"(by) : "f"(b.y));
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int g = 0; g < GR; g++) {
+          fma2(acc[2 * g][2 * h], a[g].x, bx);
+          fma2(acc[2 * g + 1][2 * h], a[g].y, bx);
+          fma2(acc[2 * g][2 * h + 1], a[g].x, by);
+          fma2(acc[2 * g + 1][2 * h + 1], a[g].y, by);
+        }
+      }
     }
-    __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int r = r0 + tx + 16 * i;
-    if (r >= M) continue;
+  for (int c = 0; c < CPT; c++) {
+    const int col = c0 + warp * 4 * CPT + 8 * (c >> 1) + 2 * ly + (c & 1);
+    if (col >= N) continue;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int c = c0 + ty + 16 * j;
-      if (c < N) C[r + c * ldc] = acc[i][j];
+    for (int g = 0; g < GR; g++) {
+      const int r = r0 + 32 * g + lx * 4;
+      float v[4];
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[2 * g][c]));
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[2 * g + 1][c]));
+      // four consecutive rows, which are consecutive outputs but where a plane of the y-transform ends
+      float* o = XT ? C + long(col) * nx + r : C + long(r / nx) * pl + long(col) * nx + r % nx;
+      if (r + 3 < M && (reinterpret_cast<uintptr_t>(o) & 15) == 0 && (XT || r % nx + 3 < nx)) {
+        *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+          if (r + e < M) (XT ? C + long(col) * nx : C + long((r + e) / nx) * pl + long(col) * nx)[XT ? r + e : (r + e) % nx] = v[e];
+      }
     }
   }
 }
@@ -74,33 +165,84 @@ __global__ void __launch_bounds__(256) k_gemm_f32(int M, int N, int K, const flo
 // ---------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ bool low_mode(int l, int m) { return l < 2 && m < 2; }
 
-template <int NZ>
-__global__ void __launch_bounds__(128) k_tri_f32(int nx, int ny, const float* __restrict__ lam, const float4* __restrict__ zop,
-                                                 float* __restrict__ hat) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (l >= nx || low_mode(l, m)) return;
-  const float shift = __ldg(lam + l) + __ldg(lam + nx + m);
+// One thread per mode, 64 modes in l per block. The column stays in shared memory between the sweeps (c' and d of every
+// level, 512 nz bytes per block), so T2 is read once and written once, and a batch of levels is loaded ahead of the
+// recurrence, whose two IEEE divisions per level are the rest of the time. The lowest 2 x 2 modes run in FP64 in their
+// own threads of the same launch, their columns in cpd. 464 x 464 x 60: 61 us against 69 us for a kernel that kept c' and
+// the column in global memory plus 47 us for the lowest modes in a launch of their own.
+constexpr int kTriThreads = 64, kTriBatch = 16, kTriSmemLevels = 440;   // 440 levels: 220 KB
+__global__ void __launch_bounds__(kTriThreads) k_tri_f32(int nx, int ny, int nz, const float* __restrict__ lam,
+                                                         const float4* __restrict__ zop, float* __restrict__ hat,
+                                                         double* __restrict__ cpd) {
+  extern __shared__ float tsm[];
+  const int l = blockIdx.x * kTriThreads + threadIdx.x, m = blockIdx.y;
+  if (l >= nx) return;
   const long sxy = long(nx) * ny;
   float* h = hat + l + long(nx) * m;
-  float cp[NZ];
-  float cprev = 0.f, dprev = 0.f;
+  float hv[kTriBatch], hn[kTriBatch];   // the batch being swept, the next one in flight
+  auto fetch = [&](float (&to)[kTriBatch], int k0) {
 #pragma unroll
-  for (int k = 0; k < NZ; k++) {
-    const float4 o = __ldg(zop + k);
-    const float den = o.z + shift * o.w - o.x * cprev;
-    cprev = o.y / den;
-    dprev = (h[sxy * k] - o.x * dprev) / den;
-    cp[k] = cprev;
-    h[sxy * k] = dprev;
+    for (int u = 0; u < kTriBatch; u++) to[u] = k0 + u < nz ? h[sxy * (k0 + u)] : 0.f;
+  };
+  auto advance = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < kTriBatch; u++) hv[u] = hn[u];
+    fetch(hn, k0 + kTriBatch);
+  };
+  fetch(hn, 0);
+  if (low_mode(l, m)) {
+    const double shift = double(lam[l]) + double(lam[nx + m]);
+    double* cp = cpd + (m * 2 + l) * nz;
+    double* dd = cpd + 4 * nz + (m * 2 + l) * nz;
+    double cprev = 0.0, dprev = 0.0;
+    for (int k0 = 0; k0 < nz; k0 += kTriBatch) {
+      advance(k0);
+#pragma unroll
+      for (int u = 0; u < kTriBatch; u++) {
+        if (k0 + u >= nz) break;
+        const float4 o = __ldg(zop + k0 + u);
+        const double den = double(o.z) + shift * double(o.w) - double(o.x) * cprev;
+        cprev = double(o.y) / den;
+        dprev = (double(hv[u]) - double(o.x) * dprev) / den;
+        cp[k0 + u] = cprev;
+        dd[k0 + u] = dprev;
+      }
+    }
+    double above = dprev;
+    h[sxy * (nz - 1)] = float(above);
+#pragma unroll 8
+    for (int k = nz - 2; k >= 0; k--) {
+      above = dd[k] - cp[k] * above;
+      h[sxy * k] = float(above);
+    }
+    return;
+  }
+  const float shift = __ldg(lam + l) + __ldg(lam + nx + m);
+  float* cp = tsm + threadIdx.x;
+  float* d = cp + nz * kTriThreads;
+  float cprev = 0.f, dprev = 0.f;
+  for (int k0 = 0; k0 < nz; k0 += kTriBatch) {
+    advance(k0);
+#pragma unroll
+    for (int u = 0; u < kTriBatch; u++) {
+      if (k0 + u >= nz) break;
+      const float4 o = __ldg(zop + k0 + u);
+      const float den = o.z + shift * o.w - o.x * cprev;
+      cprev = o.y / den;
+      dprev = (hv[u] - o.x * dprev) / den;
+      cp[(k0 + u) * kTriThreads] = cprev;
+      d[(k0 + u) * kTriThreads] = dprev;
+    }
   }
   float above = dprev;
-#pragma unroll
-  for (int k = NZ - 2; k >= 0; k--) {
-    above = h[sxy * k] - cp[k] * above;
+  h[sxy * (nz - 1)] = above;
+#pragma unroll 4
+  for (int k = nz - 2; k >= 0; k--) {
+    above = d[k * kTriThreads] - cp[k * kTriThreads] * above;
     h[sxy * k] = above;
   }
 }
-// any nz: forward-sweep coefficients in a global scratch column
+// columns too long for shared memory: forward-sweep coefficients in a global scratch column
 __global__ void k_tri_f32_any(int nx, int ny, int nz, const float* __restrict__ lam, const float4* __restrict__ zop,
                               float* __restrict__ hat, float* __restrict__ cpbuf) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
@@ -124,7 +266,7 @@ __global__ void k_tri_f32_any(int nx, int ny, int nz, const float* __restrict__ 
     h[sxy * k] = above;
   }
 }
-// the lowest 2 x 2 modes in FP64 (one warp)
+// their lowest 2 x 2 modes in FP64 (one warp)
 __global__ void k_tri_f64_low(int nx, int ny, int nz, const float* __restrict__ lam, const float4* __restrict__ zop,
                               float* __restrict__ hat, double* __restrict__ cpbuf) {
   const int t = threadIdx.x;
@@ -163,6 +305,8 @@ static int ck(cudaError_t e, const char* what) {
   return OB_OK;
 }
 
+static void fp32_attrs();
+
 int PoissonPlan::create(int nx_, int ny_, int nz_, double dx_, double dz_, int precision_) {
   nx = nx_; ny = ny_; nz = nz_; dx = dx_; dz = dz_; precision = precision_;
   if (nx < 2 || ny < 2 || nz < 2 || nz > 4096) { set_error("poisson: bad size %d x %d x %d", nx, ny, nz); return OB_ERR_INVALID; }
@@ -191,11 +335,14 @@ int PoissonPlan::create(int nx_, int ny_, int nz_, double dx_, double dz_, int p
   if ((rc = ck(cudaMalloc(&mats, M.size() * sizeof(float)), "poisson mats"))) return rc;
   if ((rc = ck(cudaMalloc(&lam, lamh.size() * sizeof(float)), "poisson eig"))) return rc;
   if ((rc = ck(cudaMalloc(&zop, size_t(nz) * sizeof(float4)), "poisson zop"))) return rc;
-  if ((rc = ck(cudaMalloc(&tmp, n * sizeof(float)), "poisson tmp"))) return rc;
-  if ((rc = ck(cudaMalloc(&hat, n * sizeof(float)), "poisson hat"))) return rc;
-  if ((rc = ck(cudaMalloc(&cpd, size_t(8) * nz * sizeof(double)), "poisson low-mode scratch"))) return rc;
-  if (nz != 40 && nz != 80 && nz != 16) {
-    if ((rc = ck(cudaMalloc(&cpf, n * sizeof(float)), "poisson tri scratch"))) return rc;
+  if (precision == 0) {   // the tensor-core precisions hold their fields in the buffers of tc_create
+    fp32_attrs();
+    if ((rc = ck(cudaMalloc(&tmp, n * sizeof(float)), "poisson tmp"))) return rc;
+    if ((rc = ck(cudaMalloc(&hat, n * sizeof(float)), "poisson hat"))) return rc;
+    if ((rc = ck(cudaMalloc(&cpd, size_t(8) * nz * sizeof(double)), "poisson low-mode scratch"))) return rc;
+    if (nz > kTriSmemLevels) {
+      if ((rc = ck(cudaMalloc(&cpf, n * sizeof(float)), "poisson tri scratch"))) return rc;
+    }
   }
   if ((rc = ck(cudaMemcpy(mats, M.data(), M.size() * sizeof(float), cudaMemcpyHostToDevice), "poisson upload"))) return rc;
   if ((rc = ck(cudaMemcpy(lam, lamh.data(), lamh.size() * sizeof(float), cudaMemcpyHostToDevice), "poisson upload"))) return rc;
@@ -228,26 +375,40 @@ void PoissonPlan::destroy() {
   cpd = nullptr;
 }
 
+// the width of the tiles that span n outputs of a DST matrix: 96 where that pads n less than 128 does
+static bool narrow_tiles(int n) { return (n + 95) / 96 * 96 < (n + 127) / 128 * 128; }
+template <bool XT, int GR, int CPT>
+static void launch_gemm(int M, int N, int K, const float* mat, const float* src, float* dst, int nx, long pl, cudaStream_t s) {
+  const int rt = (M + 32 * GR - 1) / (32 * GR), ct = (N + 16 * CPT - 1) / (16 * CPT);
+  k_gemm_f32<XT, GR, CPT><<<unsigned(rt) * unsigned(ct), GTH, gemm_smem_bytes<GR, CPT>(), s>>>(M, N, K, mat, src, dst, nx, pl, XT ? rt : ct);
+}
+static void fp32_attrs() {
+  static bool done = false;
+  if (done) return;
+  cudaFuncSetAttribute(k_gemm_f32<true, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 8>());
+  cudaFuncSetAttribute(k_gemm_f32<true, 3, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<3, 8>());
+  cudaFuncSetAttribute(k_gemm_f32<false, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 8>());
+  cudaFuncSetAttribute(k_gemm_f32<false, 4, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 6>());
+  cudaFuncSetAttribute(k_tri_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriSmemLevels * kTriThreads * 8);
+  done = true;
+}
 // x-transform (solver.js mode 0): dst(l, col) = sum_i M(l, i) src(i, col), col = j + ny k
 void PoissonPlan::gemm_x(const float* Mx, const float* src, float* dst, cudaStream_t s) const {
-  const int cols = ny * nz;
-  dim3 grid((nx + GBM - 1) / GBM, (cols + GBN - 1) / GBN, 1);
-  k_gemm_f32<<<grid, 256, 0, s>>>(nx, cols, nx, Mx, nx, 1, src, 1, nx, dst, nx, 0, 0, 0);
+  if (narrow_tiles(nx)) launch_gemm<true, 3, 8>(nx, ny * nz, nx, Mx, src, dst, nx, 0, s);
+  else launch_gemm<true, 4, 8>(nx, ny * nz, nx, Mx, src, dst, nx, 0, s);
 }
 // y-transform (mode 1), per plane k: dst(i, m) = sum_j src(i, j) M(m, j)
 void PoissonPlan::gemm_y(const float* My, const float* src, float* dst, cudaStream_t s) const {
-  dim3 grid((nx + GBM - 1) / GBM, (ny + GBN - 1) / GBN, nz);
   const long pl = long(nx) * ny;
-  k_gemm_f32<<<grid, 256, 0, s>>>(nx, ny, ny, src, 1, nx, My, 1, ny, dst, nx, pl, 0, pl);
+  if (narrow_tiles(ny)) launch_gemm<false, 4, 6>(nx * nz, ny, ny, My, src, dst, nx, pl, s);
+  else launch_gemm<false, 4, 8>(nx * nz, ny, ny, My, src, dst, nx, pl, s);
 }
 void PoissonPlan::tri(float* h, cudaStream_t s) const {
-  dim3 grid((nx + 127) / 128, ny, 1);
-  switch (nz) {
-    case 16: k_tri_f32<16><<<grid, 128, 0, s>>>(nx, ny, lam, zop, h); break;
-    case 40: k_tri_f32<40><<<grid, 128, 0, s>>>(nx, ny, lam, zop, h); break;
-    case 80: k_tri_f32<80><<<grid, 128, 0, s>>>(nx, ny, lam, zop, h); break;
-    default: k_tri_f32_any<<<grid, 128, 0, s>>>(nx, ny, nz, lam, zop, h, cpf); break;
+  if (nz <= kTriSmemLevels) {
+    k_tri_f32<<<dim3((nx + kTriThreads - 1) / kTriThreads, ny), kTriThreads, size_t(nz) * kTriThreads * 8, s>>>(nx, ny, nz, lam, zop, h, cpd);
+    return;
   }
+  k_tri_f32_any<<<dim3((nx + 127) / 128, ny, 1), 128, 0, s>>>(nx, ny, nz, lam, zop, h, cpf);
   k_tri_f64_low<<<1, 32, 0, s>>>(nx, ny, nz, lam, zop, h, cpd);
 }
 
