@@ -382,15 +382,13 @@ static void launch_gemm(int M, int N, int K, const float* mat, const float* src,
   const int rt = (M + 32 * GR - 1) / (32 * GR), ct = (N + 16 * CPT - 1) / (16 * CPT);
   k_gemm_f32<XT, GR, CPT><<<unsigned(rt) * unsigned(ct), GTH, gemm_smem_bytes<GR, CPT>(), s>>>(M, N, K, mat, src, dst, nx, pl, XT ? rt : ct);
 }
+// on every create: a function's attributes belong to the device that is current
 static void fp32_attrs() {
-  static bool done = false;
-  if (done) return;
   cudaFuncSetAttribute(k_gemm_f32<true, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 8>());
   cudaFuncSetAttribute(k_gemm_f32<true, 3, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<3, 8>());
   cudaFuncSetAttribute(k_gemm_f32<false, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 8>());
   cudaFuncSetAttribute(k_gemm_f32<false, 4, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 6>());
   cudaFuncSetAttribute(k_tri_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriSmemLevels * kTriThreads * 8);
-  done = true;
 }
 // x-transform (solver.js mode 0): dst(l, col) = sum_i M(l, i) src(i, col), col = j + ny k
 void PoissonPlan::gemm_x(const float* Mx, const float* src, float* dst, cudaStream_t s) const {

@@ -1,20 +1,19 @@
 // ob_radar.cu — virtual WSR-88D gate sampling for sm_100a (radar.js:41-268).
 //
-// k_radar_cut restates WGSL_R_CUT: one thread per gate (the reference packs 4 gates per thread), gates of one radial
-// along x so that neighbouring lanes sample neighbouring points of the model (250 m apart) and share L1 lines. Each
-// gate samples the model three times across the beam (beam filling), turns the hydrometeors into reflectivity,
-// radial velocity, spectrum width, ZDR, rho_hv and KDP, and stores one 8-bit Level II code per moment. The codes go
-// out as bytes: a warp stores 32 consecutive codes of a radial, which is the reference's little-endian packing of
-// 4 codes per u32 word (radar.js:229-240) written as one 32-byte sector.
+// k_radar_scan and k_radar_cut restate WGSL_R_CUT: one thread per gate (the reference packs 4 gates per thread), gates
+// of one radial along x so that neighbouring lanes sample neighbouring points of the model (250 m apart) and share L1
+// lines. Each gate samples the model three times across the beam (beam filling), turns the hydrometeors into
+// reflectivity, radial velocity, spectrum width, ZDR, rho_hv and KDP, and stores one 8-bit Level II code per moment. The
+// codes go out as bytes: a warp stores 32 consecutive codes of a radial, which is the reference's little-endian packing
+// of 4 codes per u32 word (radar.js:229-240) written as one 32-byte sector.
 //
 // k_radar_phi restates WGSL_R_PHI: PhiDP is a running fp32 sum of 2 * KDP * dr along each radial, in gate order, so
-// each radial stays sequential (a parallel scan would round differently). One warp handles 32 radials: it stages a
-// 32 x 32 tile of KDP through shared memory so the global reads and the code stores are coalesced, then every lane
-// walks its own radial through the tile.
+// each radial stays sequential (a parallel scan would round differently).
 //
 // The quantisation code() and the PhiDP accumulation use explicitly rounded fp32 operations (no FMA contraction),
 // so identical moments give bit-identical codes to the CPU restatement; the geometry and microphysics use CUDA's
 // IEEE-accurate math functions and may contract to FMA.
+#include <cmath>
 #include <cstdint>
 
 #include "ob_common.cuh"
@@ -226,12 +225,134 @@ __device__ GateOut gate(const RadarU& R, const Grid& g, const Fields& F, int par
   return G;
 }
 
-// one thread per gate: x = gate along the radial, y = radial
+// What the scan of a cut needs of its trigonometry, worked out on the host in 64 bits: the sines of the elevation at the
+// beam's three points, its cosine, and the site's up, north and east vectors in the frame (east, north, up) of the
+// projection's centre.
+struct ScanU {
+  float se, sl, su, ce;
+  float3 up, north, east;
+};
+static ScanU scan_uniforms(const RadarU& R) {
+  const double p0 = R.geo.x, p1 = R.geo.z, dl = double(R.geo.w) - double(R.geo.y), el = R.cut.x, q = 0.4 * 0.0165;
+  auto f3 = [](double x, double y, double z) { return make_float3(float(x), float(y), float(z)); };
+  ScanU S;
+  S.se = float(std::sin(el));
+  S.sl = float(std::sin(el - q));
+  S.su = float(std::sin(el + q));
+  S.ce = float(std::cos(el));
+  S.up = f3(std::cos(p1) * std::sin(dl), std::cos(p0) * std::sin(p1) - std::sin(p0) * std::cos(p1) * std::cos(dl),
+            std::sin(p0) * std::sin(p1) + std::cos(p0) * std::cos(p1) * std::cos(dl));
+  S.north = f3(-std::sin(p1) * std::sin(dl), std::cos(p0) * std::cos(p1) + std::sin(p0) * std::sin(p1) * std::cos(dl),
+               std::sin(p0) * std::cos(p1) - std::cos(p0) * std::sin(p1) * std::cos(dl));
+  S.east = f3(std::cos(dl), std::sin(p0) * std::sin(dl), -std::cos(p0) * std::sin(dl));
+  return S;
+}
+// Whether a gate can come out anything but empty: false only if gate() leaves it empty, whatever its last bits. The
+// beam's three points are worked out with vectors and short series (the ground arc d < 0.2, the angle to the centre under
+// 0.3: errors below 1e-8, so what is left is fp32 rounding, about a metre on either side), and every bound has a margin
+// many times that (25 m in the horizontal, 1 m in the vertical); the texels looked at are all that any point within it
+// interpolates. First the hydrometeor flags of the 32 x 4 bricks around (F.actQ0, as fresh as the state: the physics pass
+// and every write of the scalars remake them), then the rain, snow and graupel themselves. Out of these alone each
+// reflectivity is +0, and with no tornado about there is no debris, so the echo is below any floor.
+__device__ __forceinline__ bool may_echo(const RadarU& R, const ScanU& S, const Grid& g, const Fields& F, int ri, int gi) {
+  const float r = R.gates.z + R.gates.w * float(gi);
+  const float az = (R.cut.y + R.cut.z * float(ri)) * 0.017453293f;
+  const float dx = R.mdl.w, dz = R.mdl2.x, zAnt = R.site.z - R.mdl2.y, a = R.site.w;
+  auto height = [&](float sn) {
+    const float q = r * r + 2.f * r * a * sn;
+    return q / (sqrtf(q + a * a) + a);
+  };
+  const float h = height(S.se), zc = zAnt + h;
+  if (zc > R.mdl.z * dz - 199.f) return false;
+  const float s = a * asinf(clampf(r * S.ce / (a + h), -1.f, 1.f));
+  constexpr float RE = 6371000.f;
+  const float d = s / RE, d2 = d * d;
+  const float sd = d * (1.f - d2 * (1.f / 6.f - d2 * (1.f / 120.f))), cd = 1.f - d2 * (0.5f - d2 * (1.f / 24.f - d2 * (1.f / 720.f)));
+  float sa, ca;
+  sincosf(az, &sa, &ca);
+  const float ux = cd * S.up.x + sd * (ca * S.north.x + sa * S.east.x), uy = cd * S.up.y + sd * (ca * S.north.y + sa * S.east.y);
+  const float uz = cd * S.up.z + sd * (ca * S.north.z + sa * S.east.z);
+  const float t2 = ux * ux + uy * uy;   // sin^2 of the angle to the centre: angle / sine = asin(t) / t
+  float2 p;
+  if (d < 0.2f && t2 < 0.09f && uz > 0.f) {
+    const float k = 1.f + t2 * (1.f / 6.f + t2 * (3.f / 40.f + t2 * (15.f / 336.f + t2 * (105.f / 3456.f + t2 * (945.f / 42240.f)))));
+    p = make_float2(RE * k * ux - R.mdl2.z, RE * k * uy - R.mdl2.w);
+  } else {
+    p = gatePos(R, az, s);
+  }
+  const float ex = 25.f / dx + 0.01f, ez = 1.f / dz + 0.001f;
+  const float gx = p.x / dx, gy = p.y / dx, gz = fmaxf(zc, 5.f) / dz;
+  if (!(gx >= -ex && gy >= -ex && gz >= -ez && gx <= R.mdl.x + ex && gy <= R.mdl.y + ex && gz <= R.mdl.z + ez)) return false;
+  if (int(R.phys.w) > 0) return true;
+  const float hl = height(S.sl) + zAnt, hu = height(S.su) + zAnt;
+  const float zl = fminf(fmaxf(hl, 5.f), fmaxf(zc, 5.f)) / dz, zu = fmaxf(fmaxf(hu, 5.f), fmaxf(zc, 5.f)) / dz;
+  const int i0 = clampi(int(floorf(gx - 0.5f - ex)), 0, g.nx - 1), i1 = clampi(int(floorf(gx - 0.5f + ex)) + 1, 0, g.nx - 1);
+  const int j0 = clampi(int(floorf(gy - 0.5f - ex)), 0, g.ny - 1), j1 = clampi(int(floorf(gy - 0.5f + ex)) + 1, 0, g.ny - 1);
+  const int k0 = clampi(int(floorf(zl - 0.5f - ez)), 0, g.nz - 1), k1 = clampi(int(floorf(zu - 0.5f + ez)) + 1, 0, g.nz - 1);
+  unsigned any = 0;
+  for (int k = k0; k <= k1; k++)
+    for (int by = j0 >> 2; by <= j1 >> 2; by++)
+      for (int bx = i0 >> 5; bx <= i1 >> 5; bx++) any |= __ldg(F.actQ0 + bx + F.nbx * (by + F.nby * k));
+  if (!any) return false;
+  // the corners of a level at once: their 12 loads are in flight together (a middle row or column is rare)
+  const bool wide = i1 - i0 > 1 || j1 - j0 > 1;
+  for (int k = k0; k <= k1; k++) {
+    const int a = g.at(i0, j0, k), b = g.at(i1, j0, k), c = g.at(i0, j1, k), d = g.at(i1, j1, k);
+    unsigned bits = 0;
+#pragma unroll
+    for (int q = 3; q < 6; q++)
+      bits |= __float_as_uint(__ldg(F.Q[0][q] + a)) | __float_as_uint(__ldg(F.Q[0][q] + b)) | __float_as_uint(__ldg(F.Q[0][q] + c)) |
+              __float_as_uint(__ldg(F.Q[0][q] + d));
+    if (wide)
+      for (int j = j0; j <= j1; j++)
+        for (int i = i0; i <= i1; i++)
+#pragma unroll
+          for (int q = 3; q < 6; q++) bits |= __float_as_uint(__ldg(F.Q[0][q] + g.at(i, j, k)));
+    if (bits) return true;   // a zero of either sign adds nothing, but a -0 here only sends the gate on
+  }
+  return false;
+}
+
+// A cut in two launches. Most gates of a volume see no rain, snow or graupel in any of their three samples, so their
+// codes are all 0. k_radar_scan tells these from the others (may_echo, in 32 registers and a third of the instructions)
+// and writes them; the rest get kActive in place of their REF code, a code that no gate has (0 is empty, values start at
+// 2), and k_radar_cut works out those. Both take one thread per gate, x = gate along the radial, y = radial. The scan is
+// bound by its instructions (arithmetic of the position, issue slots 60-70 % busy), the rest by the latency of a warp's
+// gathers and powers. VCP 212 over a 256 x 256 x 40 storm field (17 cuts of 936 gates a radial): 2051 us for one launch
+// per cut over every gate, now 380 + 601 us; a texel test on gate()'s own trigonometry took 568 us. Codes are compared
+// bit for bit, and the compiler's choice of fused multiply-adds moves with the code around them, so gate() and its launch
+// stay whole: packing the active gates into full warps changed the last bit of some moments.
+constexpr uint8_t kActive = 1;
+__global__ void __launch_bounds__(128) k_radar_scan(RadarU R, ScanU S, Grid g, Fields F, uint8_t* __restrict__ out, float* __restrict__ kdp,
+                                                    float* __restrict__ mom) {
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x, ri = blockIdx.y;
+  const int ngR = int(R.gates.x), ngD = int(R.gates.y);
+  if (gi >= ngR) return;
+  const bool active = may_echo(R, S, g, F, ri, gi);
+  const size_t oR = size_t(R.offA.x) * 4 + size_t(ri) * ngR + gi;
+  out[oR] = active ? kActive : uint8_t(0);
+  if (active) return;
+  const uint32_t mask = uint32_t(R.offB.w);
+  if (gi < ngD) {
+    const size_t o = size_t(ri) * ngD + gi;
+    if (mask & 2u) out[size_t(R.offA.y) * 4 + o] = 0;
+    if (mask & 4u) out[size_t(R.offA.z) * 4 + o] = 0;
+    if (mask & 8u) out[size_t(R.offA.w) * 4 + o] = 0;
+    if (mask & 32u) out[size_t(R.offB.y) * 4 + o] = 0;
+    kdp[o] = -1.f;
+  }
+  if (mom) {
+    float* mp = mom + (size_t(ri) * ngR + gi) * 6;
+#pragma unroll
+    for (int c = 0; c < 6; c++) mp[c] = __int_as_float(0x7fc00000);
+  }
+}
 __global__ void __launch_bounds__(128) k_radar_cut(RadarU R, Grid g, Fields F, int par, const float* __restrict__ tor,
                                                    uint8_t* __restrict__ out, float* __restrict__ kdp, float* __restrict__ mom) {
   const int gi = blockIdx.x * blockDim.x + threadIdx.x, ri = blockIdx.y;
   const int ngR = int(R.gates.x), ngD = int(R.gates.y);
   if (gi >= ngR) return;
+  if (out[size_t(R.offA.x) * 4 + size_t(ri) * ngR + gi] != kActive) return;
   const GateOut G = gate(R, g, F, par, tor, ri, gi);
   const uint32_t mask = uint32_t(R.offB.w);
   out[size_t(R.offA.x) * 4 + size_t(ri) * ngR + gi] = uint8_t(G.c[0]);
@@ -250,40 +371,92 @@ __global__ void __launch_bounds__(128) k_radar_cut(RadarU R, Grid g, Fields F, i
   }
 }
 
-// PhiDP: one warp per 32 radials, 32 x 32 KDP tiles staged through shared memory (radar.js:243-268)
-__global__ void __launch_bounds__(128) k_radar_phi(RadarU R, const float* __restrict__ kdp, uint8_t* __restrict__ out) {
-  __shared__ float tile[4][32][33];
-  __shared__ uint8_t codes[4][32][36];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int r0 = (blockIdx.x * 4 + wid) * 32;
+// PhiDP (radar.js:243-268): one block per 32 radials. The sum along a radial is a chain of fp32 additions in gate order,
+// so the only serial part is kept to just that: in turn i warp 0 (lane = radial) runs the additions of chunk i over
+// increments that are already in shared memory, while the other warps turn the KDP of chunk i + 1 (fetched before they
+// do anything else) into increments and the sums of chunk i - 1 into codes. What bounds it is the latency of the chain
+// and of a turn's loads: 175 -> 18 us per cut of 720 radials x 936 gates against one warp doing all of it for 32
+// radials.
+constexpr int kPhiChunk = 96, kPhiWarps = 16, kPhiThreads = 32 * kPhiWarps;
+constexpr int kPhiSpan = kPhiChunk / 32, kPhiRows = (32 + kPhiWarps - 2) / (kPhiWarps - 1);   // rows per helping warp
+__global__ void __launch_bounds__(kPhiThreads) k_radar_phi(RadarU R, const float* __restrict__ kdp, uint8_t* __restrict__ out) {
+  constexpr unsigned kEmpty = 0xffffffffu;   // an empty gate (no addition, code 0): a NaN that no sum produces
+  __shared__ unsigned buf[3][32][kPhiChunk + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r0 = blockIdx.x * 32;
   const int nrad = int(R.cut.w), ng = int(R.gates.y), ngq = (ng / 4) * 4;
-  if (r0 >= nrad) return;
   const float gw = R.gates.w;
-  float acc = R.nyq.w;
   uint8_t* dst = out + size_t(R.offB.x) * 4;
-  for (int g0 = 0; g0 < ngq; g0 += 32) {
-    for (int r = 0; r < 32; r++) {
-      const int ri = r0 + r;
-      tile[wid][r][lane] = (ri < nrad && g0 + lane < ngq) ? __ldg(kdp + size_t(ri) * ng + g0 + lane) : -1.f;
-    }
-    __syncwarp();
-    const int n = min(32, ngq - g0);
-    for (int t = 0; t < n; t++) {
-      const float kd = tile[wid][lane][t];
-      uint8_t c = 0;
-      if (kd >= 0.f) {
-        acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(__fmul_rn(2.f, kd), gw), 0.001f));
-        const float ph = __fsub_rn(acc, __fmul_rn(360.f, floorf(__fdiv_rn(acc, 360.f))));
-        c = uint8_t(fminf(fmaxf(rintf(__fadd_rn(__fdiv_rn(__fmul_rn(ph, 253.f), 360.f), 2.f)), 2.f), 255.f));
+  const int nch = (ngq + kPhiChunk - 1) / kPhiChunk;
+  float kd[kPhiRows][kPhiSpan];
+  // rows warp - 1, warp - 1 + 15, ... of a chunk: its KDP, its increments, its codes
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int j = 0; j < kPhiRows; j++)
+#pragma unroll
+      for (int u = 0; u < kPhiSpan; u++) {
+        const int r = warp - 1 + j * (kPhiWarps - 1), gi = c * kPhiChunk + u * 32 + lane;
+        kd[j][u] = (r < 32 && r0 + r < nrad && gi < ngq) ? __ldg(kdp + size_t(r0 + r) * ng + gi) : -1.f;
       }
-      codes[wid][lane][t] = c;
+  };
+  auto increments = [&](int c) {
+#pragma unroll
+    for (int j = 0; j < kPhiRows; j++)
+#pragma unroll
+      for (int u = 0; u < kPhiSpan; u++) {
+        const int r = warp - 1 + j * (kPhiWarps - 1);
+        const float k = kd[j][u];
+        if (r < 32) buf[c % 3][r][u * 32 + lane] = k >= 0.f ? __float_as_uint(__fmul_rn(__fmul_rn(__fmul_rn(2.f, k), gw), 0.001f)) : kEmpty;
+      }
+  };
+  auto encode = [&](int c) {
+#pragma unroll
+    for (int j = 0; j < kPhiRows; j++)
+#pragma unroll
+      for (int u = 0; u < kPhiSpan; u++) {
+        const int r = warp - 1 + j * (kPhiWarps - 1), gi = c * kPhiChunk + u * 32 + lane;
+        if (r >= 32 || r0 + r >= nrad || gi >= ngq) continue;
+        const unsigned b = buf[c % 3][r][u * 32 + lane];
+        uint8_t code = 0;
+        if (b != kEmpty) {
+          const float acc = __uint_as_float(b);
+          const float ph = __fsub_rn(acc, __fmul_rn(360.f, floorf(__fdiv_rn(acc, 360.f))));
+          code = uint8_t(fminf(fmaxf(rintf(__fadd_rn(__fdiv_rn(__fmul_rn(ph, 253.f), 360.f), 2.f)), 2.f), 255.f));
+        }
+        dst[size_t(r0 + r) * ng + gi] = code;
+      }
+  };
+  if (warp > 0) {
+    fetch(0);
+    increments(0);
+  }
+  __syncthreads();
+  float acc = R.nyq.w;
+  for (int i = 0; i <= nch; i++) {
+    if (warp == 0) {
+      if (i < nch) {
+        unsigned* row = buf[i % 3][lane];
+        for (int t0 = 0; t0 < kPhiChunk; t0 += 32) {
+          unsigned b[32];
+#pragma unroll
+          for (int t = 0; t < 32; t++) b[t] = row[t0 + t];
+#pragma unroll
+          for (int t = 0; t < 32; t++) {
+            const float next = __fadd_rn(acc, __uint_as_float(b[t]));
+            const bool empty = b[t] == kEmpty;
+            acc = empty ? acc : next;
+            b[t] = empty ? kEmpty : __float_as_uint(acc);
+          }
+#pragma unroll
+          for (int t = 0; t < 32; t++) row[t0 + t] = b[t];
+        }
+      }
+    } else {
+      if (i + 1 < nch) fetch(i + 1);
+      if (i > 0) encode(i - 1);
+      if (i + 1 < nch) increments(i + 1);
     }
-    __syncwarp();
-    for (int r = 0; r < 32; r++) {
-      const int ri = r0 + r;
-      if (ri < nrad && lane < n) dst[size_t(ri) * ng + g0 + lane] = codes[wid][r][lane];
-    }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
@@ -292,8 +465,9 @@ __global__ void __launch_bounds__(128) k_radar_phi(RadarU R, const float* __rest
 void launch_radar_cut(const RadarU& R, const Grid& g, const Fields& F, int par, const float* tor, uint8_t* out, float* kdp,
                       float* mom, cudaStream_t s) {
   const int ngR = int(R.gates.x), nrad = int(R.cut.w);
+  k_radar_scan<<<dim3((ngR + 127) / 128, nrad), 128, 0, s>>>(R, scan_uniforms(R), g, F, out, kdp, mom);
   k_radar_cut<<<dim3((ngR + 127) / 128, nrad), 128, 0, s>>>(R, g, F, par, tor, out, kdp, mom);
-  if (uint32_t(R.offB.w) & 16u) k_radar_phi<<<(nrad + 127) / 128, 128, 0, s>>>(R, kdp, out);
+  if (uint32_t(R.offB.w) & 16u) k_radar_phi<<<(nrad + 31) / 32, kPhiThreads, 0, s>>>(R, kdp, out);
 }
 
 }  // namespace ob
