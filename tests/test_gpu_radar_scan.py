@@ -69,7 +69,7 @@ def test_phidp_chain(oracle_lib, native, nrad, ngd):
     m.set_field(N.FIELD_Q1, q1)
     m.set_field(N.FIELD_Q2, q2)
     geo = RD.Geo(35.9, -97.2, 48000.0, 40000.0, 300.0)
-    lat, lon = geo.from_model(24000.0, 20000.0)
+    lat, lon = geo.from_model(500.0, 20000.0)   # in light rain, and the domain reaches 196 Doppler gates from it
     sim = RD.RadarSim(m, geo, seed=3)
     R = sim.add_radar({"id": "KTST", "lat": lat, "lon": lon, "h": 305.0}, {"vcp": 212})
     R["vol"], R["az0"] = 1, 0.61
