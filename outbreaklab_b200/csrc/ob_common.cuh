@@ -58,11 +58,12 @@ struct Fields {
   const float* bnd; // OB_MAX_BOUNDS x 148
   const float* ci;  // events x 12
   unsigned int* flags;  // [0] NaN/Inf counter
-  // clear-air skip of the hydrometeor channels, per brick of 32 x 4 x 1 cells (nbx x nby x nz bricks)
-  unsigned int* actQ0;   // Q slot 0 holds a hydrometeor or a nonzero spare channel in the brick
-  unsigned int* actQt;   // the advection scratch Qt holds one (its block computed them)
-  unsigned int* zeroQt;  // the scratch's hydrometeor and spare channels are known to be zero there
-  unsigned int* zeroQ1;  // Q slot 1's hydrometeor and spare channels are known to be zero there
+  // skip of absent hydrometeor and spare channels, per brick of 32 x 4 x 1 cells (nbx x nby x nz bricks): bit c of a
+  // flag word stands for channel c (1..7)
+  unsigned int* actQ0;   // Q slot 0 may hold the channel in the brick
+  unsigned int* actQt;   // the advection scratch Qt may hold it (its block computed it)
+  unsigned int* zeroQt;  // the scratch's channel is known to be zero there
+  unsigned int* zeroQ1;  // Q slot 1's channel is known to be zero there
   int nbx, nby;
   float fallmax;         // bound on every hydrometeor fall speed of the base state (m/s)
   // sponge coefficients tabulated once per parameter set (k_tables): spz[2k] = top sponge at the cell centre height

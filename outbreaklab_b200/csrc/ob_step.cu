@@ -523,21 +523,36 @@ __device__ __forceinline__ float2 minmaxQ(const float* __restrict__ f, const Tap
                      fmaxf(fmaxf(fmaxf(a, b), fmaxf(c, d)), fmaxf(fmaxf(e, h), fmaxf(k, l))));
 }
 
-// Clear-air skip of the hydrometeor channels (qc, qi, qr, qs, qg, Nr) and of the spare fourth Q2 channel, which no
-// scheme sets and physics only carries. A block (one brick of 32 x 4 x 1 cells) reads those channels only inside the
-// footprints of its departure points; if every brick touching that region holds none of them (a hydrometeor or a
-// nonzero spare), the semi-Lagrangian samples, the MacCormack correction, the limiter and the clip all give exactly
-// +0, so the block writes zeros (once) instead of gathering. Falling hydrometeors shift a departure point vertically by
-// at most dt/dz * fallmax, which widens the region in z.
+// Skip of the hydrometeor channels (qc, qi, qr, qs, qg, Nr) and of the spare fourth Q2 channel (which no scheme sets and
+// physics only carries) where they are absent. A block (one brick of 32 x 4 x 1 cells) reads a channel only inside the
+// footprints of its departure points; if no brick touching that region holds it (the flags below keep one bit per
+// channel), the semi-Lagrangian sample, the MacCormack correction, the limiter and the clip all give exactly +0, so the
+// block writes zeros (once) instead of gathering. Falling hydrometeors shift a departure point vertically by at most
+// dt/dz * fallmax, which widens the region in z. One bit per channel and not one per brick, because most bricks of a
+// storm hold some species only (an anvil is ice and snow, a warm shower cloud and rain, the Lin scheme never sets Nr and
+// the spare): 640 x 640 x 40 with a storm every 60 km, ADVQ1 396 -> 335 us, ADVQ2 842 -> 631 us.
+constexpr unsigned kHydro = 0xfeu;   // bits of the hydrometeor and spare channels, 1..7
+// the bits that any thread of a 128-thread block sets, in every thread
+__device__ __forceinline__ unsigned block_or(unsigned v) {
+  __shared__ unsigned w[4];
+  const int t = threadIdx.x + blockDim.x * threadIdx.y;
+  v = __reduce_or_sync(0xffffffffu, v);
+  if ((t & 31) == 0) w[t >> 5] = v;
+  __syncthreads();
+  return w[0] | w[1] | w[2] | w[3];
+}
 struct Region {
   int x0, x1, y0, y1, z0, z1;
 };
-__device__ __forceinline__ bool region_active(const Grid& g, const Fields& F, Region r, const unsigned int* flagsA,
-                                              const unsigned int* flagsB) {
+// the channels that a brick touching the block's region holds (bits 1..7), the same for all threads of the block
+__device__ __forceinline__ unsigned region_channels(const Grid& g, const Fields& F, Region r, const unsigned int* flagsA,
+                                                    const unsigned int* flagsB) {
   __shared__ int red[6];
+  __shared__ unsigned held;
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     red[0] = red[2] = red[4] = 1 << 30;
     red[1] = red[3] = red[5] = -(1 << 30);
+    held = 0u;
   }
   __syncthreads();
   // warp-level min/max, then one shared atomic per warp
@@ -564,7 +579,10 @@ __device__ __forceinline__ bool region_active(const Grid& g, const Fields& F, Re
     any |= __ldg(flagsA + b);
     if (flagsB) any |= __ldg(flagsB + b);
   }
-  return __syncthreads_or(any != 0u) != 0;
+  any = __reduce_or_sync(m, any);
+  if ((threadIdx.x & 31) == 0 && any) atomicOr(&held, any);
+  __syncthreads();
+  return held;
 }
 
 // ---- ADVQ1 (model.js:500-529): semi-Lagrangian step of the 8 scalars, channels grouped by the fall speed of
@@ -588,40 +606,50 @@ __device__ __forceinline__ void advq1_body(const Grid& g, const Uni& U, const Fi
     r.z0 = min(r.z0, int(floorf(z - 0.5f)));
     r.z1 = max(r.z1, int(floorf(fminf(z + kk[2] * F.fallmax, float(g.nz) - 0.5f) - 0.5f)) + 1);
   }
-  const bool active = region_active(g, F, r, F.actQ0, nullptr);
   const int brick = BX + F.nbx * (BY + F.nby * BZ);
+  const unsigned zeros = F.zeroQt[brick];   // read by every thread before the barriers of the region, written after them
+  const unsigned act = region_channels(g, F, r, F.actQ0, nullptr);
+  auto has = [&](int c) { return ((act >> c) & 1u) != 0u; };
   if (in) {
     const Tap t0 = tapQ(g, x, y, z);
     F.Qt[0][o] = gatherQ(F.Q[0][0], t0);
-    if (active) {
-      F.Qt[1][o] = gatherQ(F.Q[0][1], t0);
-      F.Qt[2][o] = gatherQ(F.Q[0][2], t0);
-      F.Qt[7][o] = gatherQ(F.Q[0][7], t0);
-      const float nr0 = gatherQ(F.Q[0][6], t0);
+    if (act) {
       const Fall fl{U.step.z, U.micro2.z > 0.5f};
+      if (has(1)) F.Qt[1][o] = gatherQ(F.Q[0][1], t0);
+      if (has(2)) F.Qt[2][o] = gatherQ(F.Q[0][2], t0);
+      if (has(7)) F.Qt[7][o] = gatherQ(F.Q[0][7], t0);
+      if (has(6) && !fl.thm) F.Qt[6][o] = gatherQ(F.Q[0][6], t0);
       const float rho = bsA(F.B, g.nz, ck).z;
-      const float2 fv = fl.vtRain(__ldg(F.Q[0][3] + o), __ldg(F.Q[0][6] + o), rho);
-      const float fs = fl.vtS(__ldg(F.Q[0][4] + o), rho), fg = fl.vtGrau(__ldg(F.Q[0][5] + o), rho);
-      traceQ(g, kk, p, v, fv.x, 1.f, x, y, z);
-      F.Qt[3][o] = gatherQ(F.Q[0][3], tapQ(g, x, y, z));
-      traceQ(g, kk, p, v, fs, 1.f, x, y, z);
-      F.Qt[4][o] = gatherQ(F.Q[0][4], tapQ(g, x, y, z));
-      traceQ(g, kk, p, v, fg, 1.f, x, y, z);
-      F.Qt[5][o] = gatherQ(F.Q[0][5], tapQ(g, x, y, z));
-      if (fl.thm) {
-        traceQ(g, kk, p, v, fv.y, 1.f, x, y, z);
-        F.Qt[6][o] = gatherQ(F.Q[0][6], tapQ(g, x, y, z));
-      } else {
-        F.Qt[6][o] = nr0;
+      if (has(3) || (has(6) && fl.thm)) {
+        const float2 fv = fl.vtRain(__ldg(F.Q[0][3] + o), __ldg(F.Q[0][6] + o), rho);
+        if (has(3)) {
+          traceQ(g, kk, p, v, fv.x, 1.f, x, y, z);
+          F.Qt[3][o] = gatherQ(F.Q[0][3], tapQ(g, x, y, z));
+        }
+        if (has(6) && fl.thm) {
+          traceQ(g, kk, p, v, fv.y, 1.f, x, y, z);
+          F.Qt[6][o] = gatherQ(F.Q[0][6], tapQ(g, x, y, z));
+        }
       }
-    } else if (!F.zeroQt[brick]) {
+      if (has(4)) {
+        traceQ(g, kk, p, v, fl.vtS(__ldg(F.Q[0][4] + o), rho), 1.f, x, y, z);
+        F.Qt[4][o] = gatherQ(F.Q[0][4], tapQ(g, x, y, z));
+      }
+      if (has(5)) {
+        traceQ(g, kk, p, v, fl.vtGrau(__ldg(F.Q[0][5] + o), rho), 1.f, x, y, z);
+        F.Qt[5][o] = gatherQ(F.Q[0][5], tapQ(g, x, y, z));
+      }
+    }
+    const unsigned clear = kHydro & ~act & ~zeros;
+    if (clear) {
 #pragma unroll
-      for (int c = 1; c < 8; c++) F.Qt[c][o] = 0.f;
+      for (int c = 1; c < 8; c++)
+        if ((clear >> c) & 1u) F.Qt[c][o] = 0.f;
     }
   }
   if (threadIdx.x == 0 && threadIdx.y == 0) {
-    F.actQt[brick] = active ? 1u : 0u;
-    F.zeroQt[brick] = active ? 0u : 1u;
+    F.actQt[brick] = act;
+    F.zeroQt[brick] = kHydro & ~act;
   }
 }
 __global__ void __launch_bounds__(128, 12) k_advq1(Grid g, Uni U, Fields F, int par) { advq1_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
@@ -663,54 +691,56 @@ __device__ __forceinline__ void advq2_body(const Grid& g, const Uni& U, const Fi
     r.z0 = min(r.z0, int(floorf(fmaxf(fminf(zb, zf) - dzf, 0.5f) - 0.5f)));
     r.z1 = max(r.z1, int(floorf(fminf(fmaxf(zb, zf) + dzf, float(g.nz) - 0.5f) - 0.5f)) + 1);
   }
-  const bool active = region_active(g, F, r, F.actQ0, F.actQt);
   const int brick = BX + F.nbx * (BY + F.nby * BZ);
+  const unsigned zeros = F.zeroQ1[brick];   // read by every thread before the barriers of the region, written after them
+  const unsigned act = region_channels(g, F, r, F.actQ0, F.actQt);
+  auto has = [&](int c) { return ((act >> c) & 1u) != 0u; };
   if (in) {
     const float cx = v[0] * kk[0], cy = v[1] * kk[1], cz = v[2] * kk[2];
     const float cour = sqrtf(cx * cx + cy * cy + cz * cz);
     const float sm = 0.5f * U.misc.y * clampf(cour / 0.35f, U.dzv.w, 1.f);
-    {  // the air-speed group: qv always; qc, qi and the spare channel where active
+    const Fall fl{U.step.z, U.micro2.z > 0.5f};
+    {  // the air-speed group: qv always; qc, qi, the spare channel and, in the Lin scheme, Nr where held
       const Tap tb = tapQ(g, xb, yb, zb), tf = tapQ(g, xf, yf, zf);
-      {
-        const float b = gatherQ(F.Qt[0], tb);
-        const float rr = __ldg(F.Qt[0] + o) + sm * (__ldg(F.Q[0][0] + o) - b);
-        const float2 m = minmaxQ(F.Q[0][0], tf);
-        F.Q[1][0][o] = fmaxf(clampf(rr, m.x, m.y), 0.f);
-      }
-      if (active) {
-        const Fall fl{U.step.z, U.micro2.z > 0.5f};
-        constexpr int kAir[3] = {1, 2, 7};  // qc, qi, spare
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          const int c = kAir[i];
-          const float b = gatherQ(F.Qt[c], tb);
-          const float rr = __ldg(F.Qt[c] + o) + sm * (__ldg(F.Q[0][c] + o) - b);
-          const float2 m = minmaxQ(F.Q[0][c], tf);
-          F.Q[1][c][o] = fmaxf(clampf(rr, m.x, m.y), 0.f);
-        }
-        if (!fl.thm) {
-          const float b = gatherQ(F.Qt[6], tb);
-          const float rr = __ldg(F.Qt[6] + o) + sm * (__ldg(F.Q[0][6] + o) - b);
-          const float2 m = minmaxQ(F.Q[0][6], tf);
-          F.Q[1][6][o] = fmaxf(clampf(rr, m.x, m.y), 0.f);
-        }
+      auto air = [&](int c) {
+        const float b = gatherQ(F.Qt[c], tb);
+        const float rr = __ldg(F.Qt[c] + o) + sm * (__ldg(F.Q[0][c] + o) - b);
+        const float2 m = minmaxQ(F.Q[0][c], tf);
+        F.Q[1][c][o] = fmaxf(clampf(rr, m.x, m.y), 0.f);
+      };
+      air(0);
+      if (act) {
+        if (has(1)) air(1);
+        if (has(2)) air(2);
+        if (has(7)) air(7);
+        if (has(6) && !fl.thm) air(6);
       }
     }
-    if (active) {
-      const Fall fl{U.step.z, U.micro2.z > 0.5f};
+    if (act & 0x78u) {
       const float rho = bsA(F.B, g.nz, ck).z;
-      const float q3 = __ldg(F.Q[0][3] + o), q4 = __ldg(F.Q[0][4] + o), q5 = __ldg(F.Q[0][5] + o), q6 = __ldg(F.Q[0][6] + o);
-      const float2 fv = fl.vtRain(q3, q6, rho);
-      F.Q[1][3][o] = advq2_channel(F, g, kk, p, v, fv.x, sm, q3, 3, o);
-      F.Q[1][4][o] = advq2_channel(F, g, kk, p, v, fl.vtS(q4, rho), sm, q4, 4, o);
-      F.Q[1][5][o] = advq2_channel(F, g, kk, p, v, fl.vtGrau(q5, rho), sm, q5, 5, o);
-      if (fl.thm) F.Q[1][6][o] = advq2_channel(F, g, kk, p, v, fv.y, sm, q6, 6, o);
-    } else if (!F.zeroQ1[brick]) {
+      if (has(3) || (has(6) && fl.thm)) {
+        const float q3 = __ldg(F.Q[0][3] + o), q6 = __ldg(F.Q[0][6] + o);
+        const float2 fv = fl.vtRain(q3, q6, rho);
+        if (has(3)) F.Q[1][3][o] = advq2_channel(F, g, kk, p, v, fv.x, sm, q3, 3, o);
+        if (has(6) && fl.thm) F.Q[1][6][o] = advq2_channel(F, g, kk, p, v, fv.y, sm, q6, 6, o);
+      }
+      if (has(4)) {
+        const float q4 = __ldg(F.Q[0][4] + o);
+        F.Q[1][4][o] = advq2_channel(F, g, kk, p, v, fl.vtS(q4, rho), sm, q4, 4, o);
+      }
+      if (has(5)) {
+        const float q5 = __ldg(F.Q[0][5] + o);
+        F.Q[1][5][o] = advq2_channel(F, g, kk, p, v, fl.vtGrau(q5, rho), sm, q5, 5, o);
+      }
+    }
+    const unsigned clear = kHydro & ~act & ~zeros;
+    if (clear) {
 #pragma unroll
-      for (int c = 1; c < 8; c++) F.Q[1][c][o] = 0.f;
+      for (int c = 1; c < 8; c++)
+        if ((clear >> c) & 1u) F.Q[1][c][o] = 0.f;
     }
   }
-  if (threadIdx.x == 0 && threadIdx.y == 0) F.zeroQ1[brick] = active ? 0u : 1u;
+  if (threadIdx.x == 0 && threadIdx.y == 0) F.zeroQ1[brick] = kHydro & ~act;
 }
 __global__ void __launch_bounds__(128, 10) k_advq2(Grid g, Uni U, Fields F, int par) { advq2_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(128, 9) k_advq2_grp(const uint2* __restrict__ map, int par) {
@@ -722,17 +752,17 @@ __global__ void __launch_bounds__(128, 9) k_advq2_grp(const uint2* __restrict__ 
 // flags are cleared because the host may have written anywhere
 __global__ void __launch_bounds__(128) k_activity(Grid g, Fields F) {
   const int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y, ck = blockIdx.z;
-  bool act = false;
+  unsigned act = 0u;
   if (ci < g.nx && cj < g.ny && ck < g.nz) {
     const int o = g.at(ci, cj, ck);
 #pragma unroll
-    for (int c = 1; c < 8; c++) act |= F.Q[0][c][o] != 0.f;
+    for (int c = 1; c < 8; c++) act |= F.Q[0][c][o] != 0.f ? 1u << c : 0u;
   }
-  const bool any = __syncthreads_or(act) != 0;
+  act = block_or(act);
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     const int b = blockIdx.x + F.nbx * (blockIdx.y + F.nby * blockIdx.z);
-    F.actQ0[b] = any ? 1u : 0u;
-    F.actQt[b] = 1u;
+    F.actQ0[b] = act;
+    F.actQt[b] = kHydro;
     F.zeroQt[b] = 0u;
     F.zeroQ1[b] = 0u;
   }
@@ -792,7 +822,7 @@ __device__ __forceinline__ unsigned warp_append(unsigned* ctr) {
   return base + unsigned(__popc(mask & ((1u << lane) - 1u)));
 }
 
-// one texel of the physics pass; returns whether the cell's new state holds a hydrometeor. MM: microphysics as the
+// one texel of the physics pass; returns the hydrometeor and spare channels that the cell's new state holds (bits 1..7). MM: microphysics as the
 // scheme (kMicroPlain), the scheme plus sampled (state, tendency) pairs (kMicroRecord), or queued for the surrogate
 // kernel where it can act (kMicroSurrogate).
 // Neighbour reads clamp to the edge of their texture (textureLoad with clamped coordinates, model.js:596-606): the
@@ -800,9 +830,9 @@ __device__ __forceinline__ unsigned warp_append(unsigned* ctr) {
 // [0, n-1] (Q, aux, phi_t), computed once per texel. BND: boundary air masses present (else the target state is the
 // base state, see tgtUb).
 template <bool BND, int MM, bool HUR = false>
-__device__ __forceinline__ bool phys_texel(const Grid& g, const Uni& U, const Fields& F, int par, int ci, int cj, int ck, bool dry,
-                                           bool was0) {
-  bool hyd = false;
+__device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, const Fields& F, int par, int ci, int cj, int ck, bool dry,
+                                               unsigned old) {
+  unsigned hyd = 0u;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int o = g.at(ci, cj, ck);
   const float* __restrict__ Vu = F.V[1 - par][0] + o;
@@ -1024,15 +1054,16 @@ __device__ __forceinline__ bool phys_texel(const Grid& g, const Uni& U, const Fi
         F.Q[0][0][o] = mc.qv; F.Q[0][1][o] = mc.qc; F.Q[0][2][o] = mc.qi; F.Q[0][3][o] = mc.qr;
         F.Q[0][4][o] = mc.qs; F.Q[0][5][o] = mc.qg; F.Q[0][6][o] = mc.nr; F.Q[0][7][o] = q2[3];
         out[3] = mc.T / pi0;
-        hyd = true;
+        hyd = kHydro;
         done = true;
       }
     }
     if (!done) {
       const MCell pre = mc;
-      // with every hydrometeor exactly +0 (a dry block) each process rate is zero and the block leaves the cell as it
-      // is; the saturation adjustment below still runs (a supersaturated cell condenses)
-      if (!dry) micro_processes(U, dt, p0, rho, spk.z, mc);
+      // with every hydrometeor exactly +0 each process rate is zero and the block leaves the cell as it is; the
+      // saturation adjustment below still runs (a supersaturated cell condenses)
+      if (!dry && (mc.qc > 0.f || mc.qi > 0.f || mc.qr > 0.f || mc.qs > 0.f || mc.qg > 0.f || mc.nr > 0.f))
+        micro_processes(U, dt, p0, rho, spk.z, mc);
       if (MM == kMicroRecord && surrogate_cell(pre) &&
           float(hash3i(ci, cj, ck ^ int(__float_as_uint(float(__ldg(F.clock))) * 2654435761u)) >> 8u) * (1.f / 16777216.f) < F.mlp_rate) {
         // one (state, process tendency) pair of the scheme: 12 inputs, 10 tendencies (before the saturation
@@ -1058,16 +1089,15 @@ __device__ __forceinline__ bool phys_texel(const Grid& g, const Uni& U, const Fi
       // 1 / (1 + 0) == 1 exactly: no division outside the sponge (and, in hurricane mode, the far-field decay)
       const float keep = HUR ? 1.f / (1.f + 2.f * dt * sl + dt * envDecay) : (sl > 0.f ? 1.f / (1.f + 2.f * dt * sl) : 1.f);
       qc *= keep; qi *= keep; qr *= keep; qs *= keep; qg *= keep; nr *= keep;
-      hyd = qc > 0.f || qi > 0.f || qr > 0.f || qs > 0.f || qg > 0.f || (thm ? nr : q2[2]) > 0.f || q2[3] > 0.f;
+      const float nv[8] = {0.f, qc, qi, qr, qs, qg, thm ? nr : q2[2], q2[3]};
       F.Q[0][0][o] = fmaxf(qv, 0.f);
-      if (hyd || !was0) {  // else the channels below are zero here and slot 0 already holds zeros
-        F.Q[0][1][o] = fmaxf(qc, 0.f);
-        F.Q[0][2][o] = fmaxf(qi, 0.f);
-        F.Q[0][3][o] = fmaxf(qr, 0.f);
-        F.Q[0][4][o] = fmaxf(qs, 0.f);
-        F.Q[0][5][o] = fmaxf(qg, 0.f);
-        F.Q[0][6][o] = thm ? fmaxf(nr, 0.f) : q2[2];
-        F.Q[0][7][o] = q2[3];
+      const bool any = qc > 0.f || qi > 0.f || qr > 0.f || qs > 0.f || qg > 0.f || nv[6] > 0.f || nv[7] > 0.f;
+      if (any || old) {  // else the channels below are zero here and slot 0 already holds zeros
+#pragma unroll
+        for (int c = 1; c < 8; c++) {
+          if (nv[c] > 0.f) hyd |= 1u << c;
+          if (nv[c] > 0.f || ((old >> c) & 1u)) F.Q[0][c][o] = c == 7 ? nv[c] : fmaxf(nv[c], 0.f);
+        }
       }
       out[3] = th;
     }
@@ -1088,40 +1118,40 @@ __device__ __forceinline__ bool phys_texel(const Grid& g, const Uni& U, const Fi
 
 // The clear-air flags of a physics block (one 32 x 4 brick of cells; blocks past the last brick hold only faces, which
 // read and write no scalar), the same for all its threads: dry = Q slot 1 holds no hydrometeor and no nonzero spare in
-// the brick and its six face neighbours (ADVQ2 wrote them as zeros), which bound every scalar read of the block; was0
-// = the previous physics pass left slot 0's hydrometeor and spare channels zero in the brick (actQ0 clear), so a cell
-// whose new values there are all zero need not store them again. Hurricane mode's 2-dx filter writes slot 0 between
-// physics passes, so there was0 stays false.
+// the brick and its six face neighbours (ADVQ2 wrote them as zeros), which bound every scalar read of the block; old
+// = the hydrometeor and spare channels that the previous physics pass left in slot 0 of the brick (actQ0), so a cell
+// whose new value of another channel is zero need not store it again. Hurricane mode's 2-dx filter writes slot 0 between
+// physics passes, so there every channel counts as held.
 template <bool HUR>
-__device__ __forceinline__ void phys_flags(const Grid& g, const Fields& F, int BX, int BY, int ck, bool& dry, bool& was0) {
+__device__ __forceinline__ void phys_flags(const Grid& g, const Fields& F, int BX, int BY, int ck, bool& dry, unsigned& old) {
   dry = false;
-  was0 = false;
+  old = kHydro;
   if (BX >= F.nbx || BY >= F.nby || ck >= g.nz) return;
   const int lane = threadIdx.x & 31;
-  unsigned z = 1u;
+  unsigned z = kHydro;
   if (lane < 7) {
     const int bx = BX + (lane == 1 ? -1 : lane == 2 ? 1 : 0), by = BY + (lane == 3 ? -1 : lane == 4 ? 1 : 0);
     const int bz = ck + (lane == 5 ? -1 : lane == 6 ? 1 : 0);
     if (bx >= 0 && bx < F.nbx && by >= 0 && by < F.nby && bz >= 0 && bz < g.nz) z = F.zeroQ1[bx + F.nbx * (by + F.nby * bz)];
   }
-  dry = __all_sync(0xffffffffu, z != 0u);
-  if (!HUR) was0 = F.actQ0[BX + F.nbx * (BY + F.nby * ck)] == 0u;
+  dry = __all_sync(0xffffffffu, z == kHydro);
+  if (!HUR) old = F.actQ0[BX + F.nbx * (BY + F.nby * ck)];
 }
 
 // BND: 1 = boundary air masses present, 0 = none, -1 = decided per launch from the uniforms (U.cor.z)
 template <int MM, bool HUR = false, int BND = -1>
 __device__ __forceinline__ void phys_body(const Grid& g, const Uni& U, const Fields& F, int par, const int BX, const int BY, const int BZ) {
   const int ci = BX * blockDim.x + threadIdx.x, cj = BY * blockDim.y + threadIdx.y, ck = BZ;
-  bool dry, was0;
-  phys_flags<HUR>(g, F, BX, BY, ck, dry, was0);
-  bool hyd = false;
+  bool dry;
+  unsigned old, hyd = 0u;
+  phys_flags<HUR>(g, F, BX, BY, ck, dry, old);
   if (ci <= g.nx && cj <= g.ny && ck <= g.nz)
-    hyd = (BND == 1 || (BND < 0 && U.cor.z > 0.5f)) ? phys_texel<BND != 0, MM, HUR>(g, U, F, par, ci, cj, ck, dry, was0)
-                                                    : phys_texel<false, MM, HUR>(g, U, F, par, ci, cj, ck, dry, was0);
-  // hydrometeor flag of this block's brick for the next step's scalar advection
-  const bool any = __syncthreads_or(hyd) != 0;
+    hyd = (BND == 1 || (BND < 0 && U.cor.z > 0.5f)) ? phys_texel<BND != 0, MM, HUR>(g, U, F, par, ci, cj, ck, dry, old)
+                                                    : phys_texel<false, MM, HUR>(g, U, F, par, ci, cj, ck, dry, old);
+  // the channels this block's brick holds, for the next step's scalar advection
+  hyd = block_or(hyd);
   if (threadIdx.x == 0 && threadIdx.y == 0 && int(BX) < F.nbx && int(BY) < F.nby && ck < g.nz)
-    F.actQ0[BX + F.nbx * (BY + F.nby * ck)] = any ? 1u : 0u;
+    F.actQ0[BX + F.nbx * (BY + F.nby * ck)] = hyd;
 }
 // one kernel per microphysics mode and per presence of boundary air masses: with one texel body per kernel, ten
 // 128-thread blocks fit on an SM at 48 registers without spilling (the surrogate with boundaries keeps nine), where the
@@ -1438,7 +1468,7 @@ __global__ void k_advv2_hur(Grid g, Uni U, Fields F, int par) {
 __device__ __forceinline__ void brick_flags_all(const Grid& g, const Fields& F, unsigned* a, unsigned* zq, unsigned* z1) {
   if (threadIdx.x == 0 && threadIdx.y == 0 && int(blockIdx.x) < F.nbx && int(blockIdx.y) < F.nby && int(blockIdx.z) < g.nz) {
     const int b = blockIdx.x + F.nbx * (blockIdx.y + F.nby * blockIdx.z);
-    if (a) a[b] = 1u;
+    if (a) a[b] = kHydro;
     if (zq) zq[b] = 0u;
     if (z1) z1[b] = 0u;
   }
