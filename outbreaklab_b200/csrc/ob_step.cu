@@ -344,8 +344,8 @@ __device__ __forceinline__ void nut_body(const Grid& g, const Uni& U, const Fiel
   }
   F.aux[1][o] = nuv;
 }
-__global__ void __launch_bounds__(128, 16) k_nut(Grid g, Uni U, Fields F, int par) { nut_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
-__global__ void k_nut_hur(Grid g, Uni U, Fields F, int par) { nut_body<true>(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void __launch_bounds__(128, 16) k_nut(Grid g, Uni U, Fields F) { nut_body(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void k_nut_hur(Grid g, Uni U, Fields F) { nut_body<true>(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(128, 12) k_nut_grp(const uint2* __restrict__ map, int par) {
   OB_GROUP_RESOLVE
   nut_body(c_members[mem].g, c_members[mem].U, c_members[mem].F, par, gbx, gby, gbz);
@@ -358,25 +358,27 @@ struct Loc {
   float vu[3], vv[3], vw[3], vc[3];
 };
 __device__ __forceinline__ Loc localVel(const Fields& F, const Grid& g, int par, int i, int j, int k) {
-  // clamp-to-edge neighbour offsets of the staggered box, once per texel
-  const int o = g.at(i, j, k);
-  const int xm = i > 0 ? -1 : 0, xp = i < g.nx ? 1 : 0;
-  const int ym = j > 0 ? -g.px : 0, yp = j < g.ny ? g.px : 0;
-  const int zm = k > 0 ? -g.plane : 0, zp = k < g.nz ? g.plane : 0;
-  const float* __restrict__ u = F.V[par][0] + o;
-  const float* __restrict__ v = F.V[par][1] + o;
-  const float* __restrict__ w = F.V[par][2] + o;
+  // clamp-to-edge neighbour offsets of the staggered box (bytes), once per texel
+  const unsigned o = 4u * unsigned(g.at(i, j, k));
+  const unsigned xm = i > 0 ? -4u : 0u, xp = i < g.nx ? 4u : 0u;
+  const unsigned px4 = 4u * unsigned(g.px), pl4 = 4u * unsigned(g.plane);
+  const unsigned ym = j > 0 ? 0u - px4 : 0u, yp = j < g.ny ? px4 : 0u;
+  const unsigned zm = k > 0 ? 0u - pl4 : 0u, zp = k < g.nz ? pl4 : 0u;
+  const float* __restrict__ u = F.V[par][0];
+  const float* __restrict__ v = F.V[par][1];
+  const float* __restrict__ w = F.V[par][2];
+  const unsigned oxm = o + xm, oxp = o + xp, oym = o + ym, oyp = o + yp, ozm = o + zm, ozp = o + zp;
   Loc L;
-  const float pu = __ldg(u), pv = __ldg(v), pw = __ldg(w);
-  const float xpu = __ldg(u + xp), ypv = __ldg(v + yp), zpw = __ldg(w + zp);
+  const float pu = ldo(u, o), pv = ldo(v, o), pw = ldo(w, o);
+  const float xpu = ldo(u, oxp), ypv = ldo(v, oyp), zpw = ldo(w, ozp);
   L.vu[0] = pu;
-  L.vu[1] = 0.25f * (__ldg(v + xm) + pv + __ldg(v + xm + yp) + ypv);
-  L.vu[2] = 0.25f * (__ldg(w + xm) + pw + __ldg(w + xm + zp) + zpw);
-  L.vv[0] = 0.25f * (__ldg(u + ym) + pu + __ldg(u + xp + ym) + xpu);
+  L.vu[1] = 0.25f * (ldo(v, oxm) + pv + ldo(v, oxm + yp) + ypv);
+  L.vu[2] = 0.25f * (ldo(w, oxm) + pw + ldo(w, oxm + zp) + zpw);
+  L.vv[0] = 0.25f * (ldo(u, oym) + pu + ldo(u, oym + xp) + xpu);
   L.vv[1] = pv;
-  L.vv[2] = 0.25f * (__ldg(w + ym) + pw + __ldg(w + ym + zp) + zpw);
-  L.vw[0] = 0.25f * (__ldg(u + zm) + pu + __ldg(u + xp + zm) + xpu);
-  L.vw[1] = 0.25f * (__ldg(v + zm) + pv + __ldg(v + yp + zm) + ypv);
+  L.vv[2] = 0.25f * (ldo(w, oym) + pw + ldo(w, oym + zp) + zpw);
+  L.vw[0] = 0.25f * (ldo(u, ozm) + pu + ldo(u, ozm + xp) + xpu);
+  L.vw[1] = 0.25f * (ldo(v, ozm) + pv + ldo(v, ozm + yp) + ypv);
   L.vw[2] = pw;
   L.vc[0] = 0.5f * (pu + xpu);
   L.vc[1] = 0.5f * (pv + ypv);
@@ -398,19 +400,20 @@ __device__ __forceinline__ float sampleVch(const float* f, const Grid& g, int ch
 
 // the departure-point sample of a channel, with the min / max of its 8 texels (ADVV2's limiter window: the
 // reference's limiter traces the same point, model.js:455-479)
-__device__ __forceinline__ void sampleVch_mm(const Fields& F, const Grid& g, int par, int ch, int o, float x, float y, float z) {
+__device__ __forceinline__ void sampleVch_mm(const Fields& F, const Grid& g, int par, int ch, unsigned o, float x, float y, float z) {
   const float ox = ch == 0 ? 0.f : 0.5f, oy = ch == 1 ? 0.f : 0.5f, oz = ch == 2 ? 0.f : 0.5f;
   float lo, hi;
-  F.Vt[ch][o] = trilerpB_mm(F.V[par][ch], g, g.nx + 1, g.ny + 1, g.nz + 1, x - ox, y - oy, z - oz, lo, hi);
-  F.Vlo[ch][o] = lo;
-  F.Vhi[ch][o] = hi;
+  const float t = trilerpB_mm(F.V[par][ch], g, g.nx + 1, g.ny + 1, g.nz + 1, x - ox, y - oy, z - oz, lo, hi);
+  sto(F.Vt[ch], o, t);
+  sto(F.Vlo[ch], o, lo);
+  sto(F.Vhi[ch], o, hi);
 }
 __device__ __forceinline__ void advv1_body(const Grid& g, const Uni& U, const Fields& F, int par, const int BX, const int BY, const int BZ) {
   OB_TEXEL_LOOP_BEGIN(g.nx, g.ny, g.nz)
   const Loc L = localVel(F, g, par, ci, cj, ck);
   const float kk[3] = {U.der.x, U.der.x, U.der.y};  // dt/dx, dt/dx, dt/dz
   const float fi = float(ci), fj = float(cj), fk = float(ck);
-  const int o = g.at(ci, cj, ck);
+  const unsigned o = 4u * unsigned(g.at(ci, cj, ck));
   float x, y, z;
   traceV(g, kk, fi, fj + 0.5f, fk + 0.5f, L.vu, 1.f, x, y, z);
   sampleVch_mm(F, g, par, 0, o, x, y, z);
@@ -421,7 +424,7 @@ __device__ __forceinline__ void advv1_body(const Grid& g, const Uni& U, const Fi
   traceV(g, kk, fi + 0.5f, fj + 0.5f, fk + 0.5f, L.vc, 1.f, x, y, z);
   sampleVch_mm(F, g, par, 3, o, x, y, z);
 }
-__global__ void k_advv1(Grid g, Uni U, Fields F, int par) { advv1_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void __launch_bounds__(128, 16) k_advv1(Grid g, Uni U, Fields F) { advv1_body(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void k_advv1_grp(const uint2* __restrict__ map, int par) {
   OB_GROUP_RESOLVE
   advv1_body(c_members[mem].g, c_members[mem].U, c_members[mem].F, par, gbx, gby, gbz);
@@ -451,18 +454,18 @@ __device__ __forceinline__ void advv2_body(const Grid& g, const Uni& U, const Fi
   const float cx = L.vc[0] * kk[0], cy = L.vc[1] * kk[1], cz = L.vc[2] * kk[2];
   const float cour = sqrtf(cx * cx + cy * cy + cz * cz);
   const float sm = 0.5f * U.misc.y * clampf(cour / 0.35f, U.dzv.w, 1.f);
-  const int o = g.at(ci, cj, ck);
+  const unsigned o = 4u * unsigned(g.at(ci, cj, ck));
 #pragma unroll
   for (int c = 0; c < 4; c++) {
     float x, y, z;
     traceV(g, kk, P[c][0], P[c][1], P[c][2], vel[c], -1.f, x, y, z);
     const float b = sampleVch(F.Vt[c], g, c, x, y, z);
-    const float hat = __ldg(F.Vt[c] + o), old = __ldg(F.V[par][c] + o);
+    const float hat = ldo(F.Vt[c], o), old = ldo(F.V[par][c], o);
     const float r = hat + sm * (old - b);
-    F.V[1 - par][c][o] = clampf(r, __ldg(F.Vlo[c] + o), __ldg(F.Vhi[c] + o));
+    sto(F.V[1 - par][c], o, clampf(r, ldo(F.Vlo[c], o), ldo(F.Vhi[c], o)));
   }
 }
-__global__ void __launch_bounds__(128, 12) k_advv2(Grid g, Uni U, Fields F, int par) { advv2_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void __launch_bounds__(128, 12) k_advv2(Grid g, Uni U, Fields F) { advv2_body(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(128, 10) k_advv2_grp(const uint2* __restrict__ map, int par) {
   OB_GROUP_RESOLVE
   advv2_body(c_members[mem].g, c_members[mem].U, c_members[mem].F, par, gbx, gby, gbz);
@@ -472,10 +475,10 @@ __global__ void __launch_bounds__(128, 10) k_advv2_grp(const uint2* __restrict__
 // scalar advection with fall speeds (model.js:482-576)
 // ---------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void cellVel(const Fields& F, const Grid& g, int par, int i, int j, int k, float v[3]) {
-  const int o = g.at(i, j, k);
-  v[0] = 0.5f * (__ldg(F.V[par][0] + o) + __ldg(F.V[par][0] + o + 1));
-  v[1] = 0.5f * (__ldg(F.V[par][1] + o) + __ldg(F.V[par][1] + o + g.px));
-  v[2] = 0.5f * (__ldg(F.V[par][2] + o) + __ldg(F.V[par][2] + o + g.plane));
+  const unsigned o = 4u * unsigned(g.at(i, j, k));
+  v[0] = 0.5f * (ldo(F.V[par][0], o) + ldo(F.V[par][0], o + 4u));
+  v[1] = 0.5f * (ldo(F.V[par][1], o) + ldo(F.V[par][1], o + 4u * unsigned(g.px)));
+  v[2] = 0.5f * (ldo(F.V[par][2], o) + ldo(F.V[par][2], o + 4u * unsigned(g.plane)));
 }
 __device__ __forceinline__ void traceQ(const Grid& g, const float k[3], const float p[3], const float v[3], float fall, float s,
                                        float& x, float& y, float& z) {
@@ -483,12 +486,9 @@ __device__ __forceinline__ void traceQ(const Grid& g, const float k[3], const fl
   y = clampf(p[1] - s * k[1] * v[1], 0.5f, float(g.ny) - 0.5f);
   z = clampf(p[2] - s * k[2] * (v[2] - fall), 0.5f, float(g.nz) - 0.5f);
 }
-// A trilinear tap on the cell-centred box: base offsets of the 2 x 2 x 2 neighbourhood (clamp-to-edge) and the
-// weights; the same footprint is the 8-texel min/max window of the MacCormack limiter (model.js:537-540).
-struct Tap {
-  int i0, i1, r00, r10, r01, r11;
-  float ax, ay, az;
-};
+// A trilinear tap on the cell-centred box: the corners of the 2 x 2 x 2 neighbourhood (clamp-to-edge) and the weights;
+// the same footprint is the 8-texel min/max window of the MacCormack limiter (model.js:537-540).
+using Tap = Corners;
 __device__ __forceinline__ Tap tapQ(const Grid& g, float x, float y, float z) {
   // x, y, z come from traceQ, clamped to [0.5, n - 0.5]: the floor indices lie in [0, n - 1], so only the upper
   // corner needs its clamp-to-edge bound
@@ -498,29 +498,23 @@ __device__ __forceinline__ Tap tapQ(const Grid& g, float x, float y, float z) {
   t.ax = tx - float(i0);
   t.ay = ty - float(j0);
   t.az = tz - float(k0);
-  const int j1 = min(j0 + 1, g.ny - 1), k1 = min(k0 + 1, g.nz - 1);
-  t.i0 = i0;
-  t.i1 = min(i0 + 1, g.nx - 1);
-  t.r00 = g.px * (j0 + g.py * k0);
-  t.r10 = g.px * (j1 + g.py * k0);
-  t.r01 = g.px * (j0 + g.py * k1);
-  t.r11 = g.px * (j1 + g.py * k1);
+  const unsigned px4 = 4u * unsigned(g.px), pl4 = 4u * unsigned(g.plane);
+  const unsigned dx4 = i0 < g.nx - 1 ? 4u : 0u, dy4 = j0 < g.ny - 1 ? px4 : 0u, dz4 = k0 < g.nz - 1 ? pl4 : 0u;
+  t.a = 4u * unsigned(i0) + px4 * unsigned(j0) + pl4 * unsigned(k0);
+  t.c = t.a + dy4;
+  t.e = t.a + dz4;
+  t.k = t.c + dz4;
+  t.b = t.a + dx4;
+  t.d = t.c + dx4;
+  t.h = t.e + dx4;
+  t.l = t.k + dx4;
   return t;
 }
-__device__ __forceinline__ float gatherQ(const float* __restrict__ f, const Tap& t) {
-  const float c00 = __ldg(f + t.r00 + t.i0) * (1.f - t.ax) + __ldg(f + t.r00 + t.i1) * t.ax;
-  const float c10 = __ldg(f + t.r10 + t.i0) * (1.f - t.ax) + __ldg(f + t.r10 + t.i1) * t.ax;
-  const float c01 = __ldg(f + t.r01 + t.i0) * (1.f - t.ax) + __ldg(f + t.r01 + t.i1) * t.ax;
-  const float c11 = __ldg(f + t.r11 + t.i0) * (1.f - t.ax) + __ldg(f + t.r11 + t.i1) * t.ax;
-  const float c0 = c00 * (1.f - t.ay) + c10 * t.ay;
-  const float c1 = c01 * (1.f - t.ay) + c11 * t.ay;
-  return c0 * (1.f - t.az) + c1 * t.az;
-}
+__device__ __forceinline__ float gatherQ(const float* __restrict__ f, const Tap& t) { return gather8(f, t); }
 __device__ __forceinline__ float2 minmaxQ(const float* __restrict__ f, const Tap& t) {
-  const float a = __ldg(f + t.r00 + t.i0), b = __ldg(f + t.r00 + t.i1), c = __ldg(f + t.r10 + t.i0), d = __ldg(f + t.r10 + t.i1);
-  const float e = __ldg(f + t.r01 + t.i0), h = __ldg(f + t.r01 + t.i1), k = __ldg(f + t.r11 + t.i0), l = __ldg(f + t.r11 + t.i1);
-  return make_float2(fminf(fminf(fminf(a, b), fminf(c, d)), fminf(fminf(e, h), fminf(k, l))),
-                     fmaxf(fmaxf(fmaxf(a, b), fmaxf(c, d)), fmaxf(fmaxf(e, h), fmaxf(k, l))));
+  const float a = ldo(f, t.a), b = ldo(f, t.b), c = ldo(f, t.c), d = ldo(f, t.d);
+  const float e = ldo(f, t.e), h = ldo(f, t.h), k = ldo(f, t.k), l = ldo(f, t.l);
+  return make_float2(min8(a, b, c, d, e, h, k, l), max8(a, b, c, d, e, h, k, l));
 }
 
 // Skip of the hydrometeor channels (qc, qi, qr, qs, qg, Nr) and of the spare fourth Q2 channel (which no scheme sets and
@@ -590,7 +584,7 @@ __device__ __forceinline__ unsigned region_channels(const Grid& g, const Fields&
 __device__ __forceinline__ void advq1_body(const Grid& g, const Uni& U, const Fields& F, int par, const int BX, const int BY, const int BZ) {
   const int ci = BX * blockDim.x + threadIdx.x, cj = BY * blockDim.y + threadIdx.y, ck = BZ;
   const bool in = ci < g.nx && cj < g.ny && ck < g.nz;
-  const int o = in ? g.at(ci, cj, ck) : 0;
+  const unsigned o = in ? 4u * unsigned(g.at(ci, cj, ck)) : 0u;
   const float kk[3] = {U.der.x, U.der.x, U.der.y};  // dt/dx, dt/dx, dt/dz
   float v[3] = {0.f, 0.f, 0.f};
   const float p[3] = {float(ci) + 0.5f, float(cj) + 0.5f, float(ck) + 0.5f};
@@ -612,39 +606,39 @@ __device__ __forceinline__ void advq1_body(const Grid& g, const Uni& U, const Fi
   auto has = [&](int c) { return ((act >> c) & 1u) != 0u; };
   if (in) {
     const Tap t0 = tapQ(g, x, y, z);
-    F.Qt[0][o] = gatherQ(F.Q[0][0], t0);
+    sto(F.Qt[0], o, gatherQ(F.Q[0][0], t0));
     if (act) {
       const Fall fl{U.step.z, U.micro2.z > 0.5f};
-      if (has(1)) F.Qt[1][o] = gatherQ(F.Q[0][1], t0);
-      if (has(2)) F.Qt[2][o] = gatherQ(F.Q[0][2], t0);
-      if (has(7)) F.Qt[7][o] = gatherQ(F.Q[0][7], t0);
-      if (has(6) && !fl.thm) F.Qt[6][o] = gatherQ(F.Q[0][6], t0);
+      if (has(1)) sto(F.Qt[1], o, gatherQ(F.Q[0][1], t0));
+      if (has(2)) sto(F.Qt[2], o, gatherQ(F.Q[0][2], t0));
+      if (has(7)) sto(F.Qt[7], o, gatherQ(F.Q[0][7], t0));
+      if (has(6) && !fl.thm) sto(F.Qt[6], o, gatherQ(F.Q[0][6], t0));
       const float rho = bsA(F.B, g.nz, ck).z;
       if (has(3) || (has(6) && fl.thm)) {
-        const float2 fv = fl.vtRain(__ldg(F.Q[0][3] + o), __ldg(F.Q[0][6] + o), rho);
+        const float2 fv = fl.vtRain(ldo(F.Q[0][3], o), ldo(F.Q[0][6], o), rho);
         if (has(3)) {
           traceQ(g, kk, p, v, fv.x, 1.f, x, y, z);
-          F.Qt[3][o] = gatherQ(F.Q[0][3], tapQ(g, x, y, z));
+          sto(F.Qt[3], o, gatherQ(F.Q[0][3], tapQ(g, x, y, z)));
         }
         if (has(6) && fl.thm) {
           traceQ(g, kk, p, v, fv.y, 1.f, x, y, z);
-          F.Qt[6][o] = gatherQ(F.Q[0][6], tapQ(g, x, y, z));
+          sto(F.Qt[6], o, gatherQ(F.Q[0][6], tapQ(g, x, y, z)));
         }
       }
       if (has(4)) {
-        traceQ(g, kk, p, v, fl.vtS(__ldg(F.Q[0][4] + o), rho), 1.f, x, y, z);
-        F.Qt[4][o] = gatherQ(F.Q[0][4], tapQ(g, x, y, z));
+        traceQ(g, kk, p, v, fl.vtS(ldo(F.Q[0][4], o), rho), 1.f, x, y, z);
+        sto(F.Qt[4], o, gatherQ(F.Q[0][4], tapQ(g, x, y, z)));
       }
       if (has(5)) {
-        traceQ(g, kk, p, v, fl.vtGrau(__ldg(F.Q[0][5] + o), rho), 1.f, x, y, z);
-        F.Qt[5][o] = gatherQ(F.Q[0][5], tapQ(g, x, y, z));
+        traceQ(g, kk, p, v, fl.vtGrau(ldo(F.Q[0][5], o), rho), 1.f, x, y, z);
+        sto(F.Qt[5], o, gatherQ(F.Q[0][5], tapQ(g, x, y, z)));
       }
     }
     const unsigned clear = kHydro & ~act & ~zeros;
     if (clear) {
 #pragma unroll
       for (int c = 1; c < 8; c++)
-        if ((clear >> c) & 1u) F.Qt[c][o] = 0.f;
+        if ((clear >> c) & 1u) sto(F.Qt[c], o, 0.f);
     }
   }
   if (threadIdx.x == 0 && threadIdx.y == 0) {
@@ -652,7 +646,7 @@ __device__ __forceinline__ void advq1_body(const Grid& g, const Uni& U, const Fi
     F.zeroQt[brick] = kHydro & ~act;
   }
 }
-__global__ void __launch_bounds__(128, 12) k_advq1(Grid g, Uni U, Fields F, int par) { advq1_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void __launch_bounds__(128, 16) k_advq1(Grid g, Uni U, Fields F) { advq1_body(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(128, 12) k_advq1_grp(const uint2* __restrict__ map, int par) {
   OB_GROUP_RESOLVE
   advq1_body(c_members[mem].g, c_members[mem].U, c_members[mem].F, par, gbx, gby, gbz);
@@ -660,11 +654,11 @@ __global__ void __launch_bounds__(128, 12) k_advq1_grp(const uint2* __restrict__
 
 // ---- ADVQ2 (model.js:530-576): MacCormack correction, limiter on the departure cell's 8 texels, clip >= 0 ----
 __device__ __forceinline__ float advq2_channel(const Fields& F, const Grid& g, const float kk[3], const float p[3], const float v[3],
-                                               float fall, float sm, float qc_, int c, int o) {
+                                               float fall, float sm, float qc_, int c, unsigned o) {
   float x, y, z;
   traceQ(g, kk, p, v, fall, -1.f, x, y, z);
   const float b = gatherQ(F.Qt[c], tapQ(g, x, y, z));
-  const float r = __ldg(F.Qt[c] + o) + sm * (qc_ - b);
+  const float r = ldo(F.Qt[c], o) + sm * (qc_ - b);
   traceQ(g, kk, p, v, fall, 1.f, x, y, z);
   const float2 m = minmaxQ(F.Q[0][c], tapQ(g, x, y, z));
   return fmaxf(clampf(r, m.x, m.y), 0.f);
@@ -673,7 +667,7 @@ __device__ __forceinline__ float advq2_channel(const Fields& F, const Grid& g, c
 __device__ __forceinline__ void advq2_body(const Grid& g, const Uni& U, const Fields& F, int par, const int BX, const int BY, const int BZ) {
   const int ci = BX * blockDim.x + threadIdx.x, cj = BY * blockDim.y + threadIdx.y, ck = BZ;
   const bool in = ci < g.nx && cj < g.ny && ck < g.nz;
-  const int o = in ? g.at(ci, cj, ck) : 0;
+  const unsigned o = in ? 4u * unsigned(g.at(ci, cj, ck)) : 0u;
   const float kk[3] = {U.der.x, U.der.x, U.der.y};  // dt/dx, dt/dx, dt/dz
   float v[3] = {0.f, 0.f, 0.f};
   const float p[3] = {float(ci) + 0.5f, float(cj) + 0.5f, float(ck) + 0.5f};
@@ -704,9 +698,9 @@ __device__ __forceinline__ void advq2_body(const Grid& g, const Uni& U, const Fi
       const Tap tb = tapQ(g, xb, yb, zb), tf = tapQ(g, xf, yf, zf);
       auto air = [&](int c) {
         const float b = gatherQ(F.Qt[c], tb);
-        const float rr = __ldg(F.Qt[c] + o) + sm * (__ldg(F.Q[0][c] + o) - b);
+        const float rr = ldo(F.Qt[c], o) + sm * (ldo(F.Q[0][c], o) - b);
         const float2 m = minmaxQ(F.Q[0][c], tf);
-        F.Q[1][c][o] = fmaxf(clampf(rr, m.x, m.y), 0.f);
+        sto(F.Q[1][c], o, fmaxf(clampf(rr, m.x, m.y), 0.f));
       };
       air(0);
       if (act) {
@@ -719,30 +713,30 @@ __device__ __forceinline__ void advq2_body(const Grid& g, const Uni& U, const Fi
     if (act & 0x78u) {
       const float rho = bsA(F.B, g.nz, ck).z;
       if (has(3) || (has(6) && fl.thm)) {
-        const float q3 = __ldg(F.Q[0][3] + o), q6 = __ldg(F.Q[0][6] + o);
+        const float q3 = ldo(F.Q[0][3], o), q6 = ldo(F.Q[0][6], o);
         const float2 fv = fl.vtRain(q3, q6, rho);
-        if (has(3)) F.Q[1][3][o] = advq2_channel(F, g, kk, p, v, fv.x, sm, q3, 3, o);
-        if (has(6) && fl.thm) F.Q[1][6][o] = advq2_channel(F, g, kk, p, v, fv.y, sm, q6, 6, o);
+        if (has(3)) sto(F.Q[1][3], o, advq2_channel(F, g, kk, p, v, fv.x, sm, q3, 3, o));
+        if (has(6) && fl.thm) sto(F.Q[1][6], o, advq2_channel(F, g, kk, p, v, fv.y, sm, q6, 6, o));
       }
       if (has(4)) {
-        const float q4 = __ldg(F.Q[0][4] + o);
-        F.Q[1][4][o] = advq2_channel(F, g, kk, p, v, fl.vtS(q4, rho), sm, q4, 4, o);
+        const float q4 = ldo(F.Q[0][4], o);
+        sto(F.Q[1][4], o, advq2_channel(F, g, kk, p, v, fl.vtS(q4, rho), sm, q4, 4, o));
       }
       if (has(5)) {
-        const float q5 = __ldg(F.Q[0][5] + o);
-        F.Q[1][5][o] = advq2_channel(F, g, kk, p, v, fl.vtGrau(q5, rho), sm, q5, 5, o);
+        const float q5 = ldo(F.Q[0][5], o);
+        sto(F.Q[1][5], o, advq2_channel(F, g, kk, p, v, fl.vtGrau(q5, rho), sm, q5, 5, o));
       }
     }
     const unsigned clear = kHydro & ~act & ~zeros;
     if (clear) {
 #pragma unroll
       for (int c = 1; c < 8; c++)
-        if ((clear >> c) & 1u) F.Q[1][c][o] = 0.f;
+        if ((clear >> c) & 1u) sto(F.Q[1][c], o, 0.f);
     }
   }
   if (threadIdx.x == 0 && threadIdx.y == 0) F.zeroQ1[brick] = kHydro & ~act;
 }
-__global__ void __launch_bounds__(128, 10) k_advq2(Grid g, Uni U, Fields F, int par) { advq2_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void __launch_bounds__(128, 10) k_advq2(Grid g, Uni U, Fields F) { advq2_body(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(128, 9) k_advq2_grp(const uint2* __restrict__ map, int par) {
   OB_GROUP_RESOLVE
   advq2_body(c_members[mem].g, c_members[mem].U, c_members[mem].F, par, gbx, gby, gbz);
@@ -1157,10 +1151,12 @@ __device__ __forceinline__ void phys_body(const Grid& g, const Uni& U, const Fie
 // 128-thread blocks fit on an SM at 48 registers without spilling (the surrogate with boundaries keeps nine), where the
 // kernel holding both bodies needed 56 registers at nine blocks; 0.64 -> 0.61 ms at 640 x 640 x 40
 template <int MM, int BND>
-__global__ void __launch_bounds__(128, (MM == kMicroSurrogate && BND == 1) ? 9 : 10) k_phys(Grid g, Uni U, Fields F, int par) {
+__global__ void __launch_bounds__(128, (MM == kMicroSurrogate && BND == 1) ? 9 : 10) k_phys(Grid g, Uni U, Fields F) {
+  constexpr int par = 0;
   phys_body<MM, false, BND>(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z);
 }
-__global__ void __launch_bounds__(128) k_phys_hur(Grid g, Uni U, Fields F, int par) {
+__global__ void __launch_bounds__(128) k_phys_hur(Grid g, Uni U, Fields F) {
+  constexpr int par = 0;
   phys_body<kMicroPlain, true>(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <int MM>
@@ -1194,7 +1190,7 @@ __device__ __forceinline__ void div_body(const Grid& g, const Uni& U, const Fiel
   }
   if (F.rhs) F.rhs[g.pidx(ci, cj, ck)] = r;  // fp32 solve, or the residual of the refined solve
 }
-__global__ void k_div(Grid g, Uni U, Fields F, int par) { div_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void k_div(Grid g, Uni U, Fields F) { div_body(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void k_div_grp(const uint2* __restrict__ map, int par) {
   OB_GROUP_RESOLVE
   div_body(c_members[mem].g, c_members[mem].U, c_members[mem].F, par, gbx, gby, gbz);
@@ -1221,7 +1217,7 @@ __device__ __forceinline__ void proj_body(const Grid& g, const Uni& U, const Fie
   F.V[1 - par][2][o] = w;
   F.V[1 - par][3][o] = __ldg(F.V[par][3] + o);
 }
-__global__ void k_proj(Grid g, Uni U, Fields F, int par) { proj_body(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z); }
+__global__ void k_proj(Grid g, Uni U, Fields F) { proj_body(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void k_proj_grp(const uint2* __restrict__ map, int par) {
   OB_GROUP_RESOLVE
   proj_body(c_members[mem].g, c_members[mem].U, c_members[mem].F, par, gbx, gby, gbz);
@@ -1249,7 +1245,8 @@ __global__ void k_rain_grp(const uint2* __restrict__ map, int par) {
 // ---------------------------------------------------------------------------------------------------------------
 // WGSL_M_MAP (model.js:1028-1100): 16 diagnostics per column
 // ---------------------------------------------------------------------------------------------------------------
-__global__ void k_maps(Grid g, Uni U, Fields F, int par, float4* out) {
+__global__ void k_maps(Grid g, Uni U, Fields F, float4* out) {
+  constexpr int par = 0;
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.nx || j >= g.ny) return;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -1376,7 +1373,8 @@ __device__ __forceinline__ void traceQH(const Uni& U, const Fields& F, const Gri
   traceQ(g, k, p, vm, fall, s, x, y, z);
 }
 
-__global__ void k_prep(Grid g, Uni U, Fields F, int par) {
+__global__ void k_prep(Grid g, Uni U, Fields F) {
+  constexpr int par = 0;
   OB_BLOCKS_DIRECT
   OB_TEXEL_LOOP_BEGIN(g.nx, g.ny, g.nz)
   auto P = [&](int a, int b, int c) {
@@ -1397,7 +1395,8 @@ __global__ void k_prep(Grid g, Uni U, Fields F, int par) {
 }
 
 // 4th-order horizontal hyperdiffusion of V and Q into V[1-par], Q slot 1 (model.js:948-994)
-__global__ void k_filt(Grid g, Uni U, Fields F, int par) {
+__global__ void k_filt(Grid g, Uni U, Fields F) {
+  constexpr int par = 0;
   OB_BLOCKS_DIRECT
   OB_TEXEL_LOOP_BEGIN(g.nx, g.ny, g.nz)
   const float a = U.hur5.z;
@@ -1421,7 +1420,8 @@ __global__ void k_filt(Grid g, Uni U, Fields F, int par) {
 }
 
 // ADVV1/2 of hurricane mode (model.js:434-481): trajectories from the true winds, values carried from Vp
-__global__ void k_advv1_hur(Grid g, Uni U, Fields F, int par) {
+__global__ void k_advv1_hur(Grid g, Uni U, Fields F) {
+  constexpr int par = 0;
   OB_BLOCKS_DIRECT
   OB_TEXEL_LOOP_BEGIN(g.nx, g.ny, g.nz)
   const Loc L = localVel(F, g, par, ci, cj, ck);
@@ -1437,7 +1437,8 @@ __global__ void k_advv1_hur(Grid g, Uni U, Fields F, int par) {
     F.Vt[c][o] = sampleVch(F.Vp[c], g, c, x, y, z);
   }
 }
-__global__ void k_advv2_hur(Grid g, Uni U, Fields F, int par) {
+__global__ void k_advv2_hur(Grid g, Uni U, Fields F) {
+  constexpr int par = 0;
   OB_BLOCKS_DIRECT
   OB_TEXEL_LOOP_BEGIN(g.nx, g.ny, g.nz)
   const Loc L = localVel(F, g, par, ci, cj, ck);
@@ -1473,7 +1474,8 @@ __device__ __forceinline__ void brick_flags_all(const Grid& g, const Fields& F, 
     if (z1) z1[b] = 0u;
   }
 }
-__global__ void k_advq1_hur(Grid g, Uni U, Fields F, int par) {
+__global__ void k_advq1_hur(Grid g, Uni U, Fields F) {
+  constexpr int par = 0;
   brick_flags_all(g, F, F.actQt, F.zeroQt, nullptr);
   const int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y, ck = blockIdx.z;
   if (ci >= g.nx || cj >= g.ny || ck >= g.nz) return;
@@ -1503,7 +1505,8 @@ __global__ void k_advq1_hur(Grid g, Uni U, Fields F, int par) {
   F.Qt[6][o] = thm ? at(fv.y, 6) : gatherQ(F.Q[0][6], t0);
   F.Qt[7][o] = gatherQ(F.Q[0][7], t0);
 }
-__global__ void k_advq2_hur(Grid g, Uni U, Fields F, int par) {
+__global__ void k_advq2_hur(Grid g, Uni U, Fields F) {
+  constexpr int par = 0;
   brick_flags_all(g, F, nullptr, nullptr, F.zeroQ1);
   const int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y, ck = blockIdx.z;
   if (ci >= g.nx || cj >= g.ny || ck >= g.nz) return;
@@ -1543,6 +1546,13 @@ __global__ void k_advq2_hur(Grid g, Uni U, Fields F, int par) {
 // ---------------------------------------------------------------------------------------------------------------
 static inline dim3 grid3(int X, int Y, int Z, dim3 b) { return dim3((X + b.x - 1) / b.x, (Y + b.y - 1) / b.y, Z); }
 static const dim3 kB3(32, 4, 1);
+// the fields with the wind slot of this parity first: a kernel over one model always reads V[0] and writes V[1] (or the
+// other way round), so that its field pointers are launch constants and not picked by an index
+static Fields facing(Fields F, int par) {
+  if (par)
+    for (int c = 0; c < 4; c++) std::swap(F.V[0][c], F.V[1][c]);
+  return F;
+}
 static const dim3 kB2(32, 8, 1);
 
 void launch_lsf(const Grid& g, const Uni& U, const Fields& F, cudaStream_t s) {
@@ -1555,32 +1565,32 @@ void launch_init(const Grid& g, const Uni& U, const Fields& F, cudaStream_t s) {
   k_init<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F);
 }
 void launch_nut(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
-  if (U.hur.x > 0.5f) k_nut_hur<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, F, par);
-  else k_nut<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, F, par);
+  if (U.hur.x > 0.5f) k_nut_hur<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, facing(F, par));
+  else k_nut<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, facing(F, par));
 }
 void launch_advv(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
   if (U.hur.x > 0.5f && F.Vp[0]) {
-    k_advv1_hur<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F, par);
-    k_advv2_hur<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F, par);
+    k_advv1_hur<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
+    k_advv2_hur<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
     return;
   }
-  k_advv1<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F, par);
-  k_advv2<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F, par);
+  k_advv1<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
+  k_advv2<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
 }
 void launch_advq(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
   if (U.hur.x > 0.5f) {
-    k_advq1_hur<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, F, par);
-    k_advq2_hur<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, F, par);
+    k_advq1_hur<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, facing(F, par));
+    k_advq2_hur<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, facing(F, par));
     return;
   }
-  k_advq1<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, F, par);
-  k_advq2<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, F, par);
+  k_advq1<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, facing(F, par));
+  k_advq2<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, facing(F, par));
 }
 void launch_prep(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
-  k_prep<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F, par);
+  k_prep<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
 }
 void launch_filt(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
-  k_filt<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F, par);
+  k_filt<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
 }
 void launch_activity(const Grid& g, const Fields& F, cudaStream_t s) {
   k_activity<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, F);
@@ -1591,33 +1601,33 @@ void launch_tables(const Grid& g, const Uni& U, const Fields& F, cudaStream_t s)
 }
 void launch_phys(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s, int micro_mode) {
   if (U.hur.x > 0.5f) {  // hurricane mode runs the scheme (model.js:578-907 with its hurricane branches)
-    k_phys_hur<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F, par);
+    k_phys_hur<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
     return;
   }
   const dim3 grid = grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3);
   const bool bnd = U.cor.z > 0.5f;
   if (micro_mode == kMicroRecord) {
-    if (bnd) k_phys<kMicroRecord, 1><<<grid, kB3, 0, s>>>(g, U, F, par);
-    else k_phys<kMicroRecord, 0><<<grid, kB3, 0, s>>>(g, U, F, par);
+    if (bnd) k_phys<kMicroRecord, 1><<<grid, kB3, 0, s>>>(g, U, facing(F, par));
+    else k_phys<kMicroRecord, 0><<<grid, kB3, 0, s>>>(g, U, facing(F, par));
   } else if (micro_mode == kMicroSurrogate) {
-    if (bnd) k_phys<kMicroSurrogate, 1><<<grid, kB3, 0, s>>>(g, U, F, par);
-    else k_phys<kMicroSurrogate, 0><<<grid, kB3, 0, s>>>(g, U, F, par);
+    if (bnd) k_phys<kMicroSurrogate, 1><<<grid, kB3, 0, s>>>(g, U, facing(F, par));
+    else k_phys<kMicroSurrogate, 0><<<grid, kB3, 0, s>>>(g, U, facing(F, par));
   } else {
-    if (bnd) k_phys<kMicroPlain, 1><<<grid, kB3, 0, s>>>(g, U, F, par);
-    else k_phys<kMicroPlain, 0><<<grid, kB3, 0, s>>>(g, U, F, par);
+    if (bnd) k_phys<kMicroPlain, 1><<<grid, kB3, 0, s>>>(g, U, facing(F, par));
+    else k_phys<kMicroPlain, 0><<<grid, kB3, 0, s>>>(g, U, facing(F, par));
   }
 }
 void launch_div(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
-  k_div<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, F, par);
+  k_div<<<grid3(g.nx, g.ny, g.nz, kB3), kB3, 0, s>>>(g, U, facing(F, par));
 }
 void launch_proj(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
-  k_proj<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, F, par);
+  k_proj<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
 }
 void launch_rain(const Grid& g, const Uni& U, const Fields& F, cudaStream_t s) {
   k_rain<<<grid3(g.nx, g.ny, 1, kB2), kB2, 0, s>>>(g, U, F);
 }
 void launch_maps(const Grid& g, const Uni& U, const Fields& F, int par, float4* out, cudaStream_t s) {
-  k_maps<<<grid3(g.nx, g.ny, 1, kB2), kB2, 0, s>>>(g, U, F, par, out);
+  k_maps<<<grid3(g.nx, g.ny, 1, kB2), kB2, 0, s>>>(g, U, facing(F, par), out);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
