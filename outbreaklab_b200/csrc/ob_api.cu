@@ -12,6 +12,7 @@
 
 #include "../../include/ob.h"
 #include "ob_common.cuh"
+#include "ob_hostcopy.cuh"
 #include "ob_mlp.cuh"
 #include "ob_poisson.cuh"
 #include "ob_radar.cuh"
@@ -266,6 +267,7 @@ static void model_free(ObModel* m) {
   if (m->ens) m->stream = m->own_stream;  // the ensemble's stream is not the model's to destroy
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
+  host_copy_release();
 }
 
 // RegionalModel.writeUniforms (model.js:1391-1425), outbreak mode
@@ -357,6 +359,7 @@ int ob_model_create(const ObGrid* grid, ObModel** out) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { set_error("ob_model_create: no CUDA device"); return OB_ERR_DEVICE; }
   ObModel* m = new ObModel();
+  host_copy_retain();
   Grid& g = m->g;
   g.nx = nx; g.ny = ny; g.nz = nz;
   g.px = ((nx + 1) + 31) / 32 * 32;
@@ -372,7 +375,7 @@ int ob_model_create(const ObGrid* grid, ObModel** out) {
   ob_params_default(&m->P);
   m->P.spongeW = float(std::fmin(std::fmax(0.08 * std::fmin(m->Lx, m->Ly), 5000.0), 40000.0));  // model.js:1207
   const double fieldsz = double(g.plane) * (nz + 1);
-  if (fieldsz * 39 * 4 > 170e9) { delete m; set_error("ob_model_create: grid too large for one GPU"); return OB_ERR_INVALID; }
+  if (fieldsz * 39 * 4 > 170e9) { delete m; host_copy_release(); set_error("ob_model_create: grid too large for one GPU"); return OB_ERR_INVALID; }
   const size_t fs = (size_t(g.plane) * (nz + 1) + 63) / 64 * 64;
   m->fs = fs;
   const size_t n2 = size_t(nx) * ny, np = size_t(g.nxp) * g.nyp * nz;
@@ -707,8 +710,7 @@ int ob_model_maps(ObModel* m, float* out) {
   if (!m || !out) { set_error("ob_model_maps: null argument"); return OB_ERR_INVALID; }
   launch_maps(m->g, m->U, m->F, m->parity, m->d_maps, m->stream);
   const size_t bytes = size_t(m->g.nx) * m->g.ny * 4 * sizeof(float4);
-  OB_TRY(cuda_status(cudaMemcpyAsync(out, m->d_maps, bytes, cudaMemcpyDeviceToHost, m->stream), "maps"));
-  return cuda_status(cudaStreamSynchronize(m->stream), "maps");
+  return cuda_status(copy_to_host(out, m->d_maps, bytes, m->stream), "maps");
 }
 
 int ob_model_tornado_candidates(ObModel* m, float zeta_min, float* out, int cap, int* count) {
@@ -762,15 +764,13 @@ int ob_model_get_field(ObModel* m, int field, void* host, size_t bytes) {
     if (bytes != need) { set_error("ob_model_get_field: %zu bytes, expected %zu", bytes, need); return OB_ERR_INVALID; }
     const void* src = field == OB_FIELD_LSF_A ? (const void*)m->F.lsfA : field == OB_FIELD_LSF_B ? (const void*)m->F.lsfB
                                                                                                  : (const void*)m->F.ciMap;
-    OB_TRY(cuda_status(cudaMemcpyAsync(host, src, bytes, cudaMemcpyDeviceToHost, m->stream), "get field"));
-    return cuda_status(cudaStreamSynchronize(m->stream), "get field");
+    return cuda_status(copy_to_host(host, src, bytes, m->stream), "get field");
   }
   if (field == OB_FIELD_PHI || field == OB_FIELD_RAIN) {
     const size_t need = field == OB_FIELD_PHI ? size_t(g.nxp) * g.nyp * g.nz * sizeof(float) : size_t(g.nx) * g.ny * sizeof(double);
     if (bytes != need) { set_error("ob_model_get_field: %zu bytes, expected %zu", bytes, need); return OB_ERR_INVALID; }
     const void* src = field == OB_FIELD_PHI ? (const void*)m->F.phi : (const void*)m->d_rain;
-    OB_TRY(cuda_status(cudaMemcpyAsync(host, src, bytes, cudaMemcpyDeviceToHost, m->stream), "get field"));
-    return cuda_status(cudaStreamSynchronize(m->stream), "get field");
+    return cuda_status(copy_to_host(host, src, bytes, m->stream), "get field");
   }
   Ptr8 p{};
   int nch, X, Y, Z;
@@ -778,8 +778,7 @@ int ob_model_get_field(ObModel* m, int field, void* host, size_t bytes) {
   const size_t need = size_t(X) * Y * Z * nch * sizeof(float);
   if (bytes != need) { set_error("ob_model_get_field: %zu bytes, expected %zu", bytes, need); return OB_ERR_INVALID; }
   launch_pack(g, p, nch, X, Y, Z, m->stage, m->stream);
-  OB_TRY(cuda_status(cudaMemcpyAsync(host, m->stage, bytes, cudaMemcpyDeviceToHost, m->stream), "get field"));
-  return cuda_status(cudaStreamSynchronize(m->stream), "get field");
+  return cuda_status(copy_to_host(host, m->stage, bytes, m->stream), "get field");
 }
 
 int ob_model_set_field(ObModel* m, int field, const void* host, size_t bytes) {
@@ -1600,6 +1599,7 @@ int ob_poisson_create(int nx, int ny, int nz, float dx, float dz, int precision,
   if (!out || precision < 0 || precision > 5) { set_error("ob_poisson_create: bad arguments"); return OB_ERR_INVALID; }
   *out = nullptr;
   ObPoisson* p = new ObPoisson();
+  host_copy_retain();
   int rc = p->plan.create(nx, ny, nz, dx, dz, precision);
   const size_t n = size_t(nx) * ny * nz * sizeof(float);
   if (rc == OB_OK) rc = cuda_status(cudaMalloc(&p->d_rhs, n), "poisson rhs");
@@ -1621,6 +1621,7 @@ int ob_poisson_destroy(ObPoisson* p) {
   if (p->d_norm) cudaFree(p->d_norm);
   if (p->stream) cudaStreamDestroy(p->stream);
   delete p;
+  host_copy_release();
   return OB_OK;
 }
 int ob_poisson_set_pair_tiles(ObPoisson* p, int on) {
@@ -1651,8 +1652,7 @@ int ob_poisson_solve(ObPoisson* p, const float* rhs, float* phi) {
   const size_t n = size_t(p->plan.nx) * p->plan.ny * p->plan.nz * sizeof(float);
   OB_TRY(cuda_status(cudaMemcpyAsync(p->d_rhs, rhs, n, cudaMemcpyHostToDevice, p->stream), "poisson upload"));
   OB_TRY(p->plan.solve(p->d_rhs, p->d_phi, p->stream));
-  OB_TRY(cuda_status(cudaMemcpyAsync(phi, p->d_phi, n, cudaMemcpyDeviceToHost, p->stream), "poisson download"));
-  OB_TRY(cuda_status(cudaStreamSynchronize(p->stream), "poisson solve"));
+  OB_TRY(cuda_status(copy_to_host(phi, p->d_phi, n, p->stream), "poisson solve"));
   return p->plan.tc_check();
 }
 int ob_poisson_time(ObPoisson* p, int reps, float* ms) {
@@ -1786,8 +1786,7 @@ int ob_radar_cut_moments(ObRadar* r, const ObRadarCut* c, float* host, size_t co
     r->mom_count = need;
   }
   OB_TRY(radar_launch(r, c, r->d_mom));
-  OB_TRY(cuda_status(cudaMemcpyAsync(host, r->d_mom, need * sizeof(float), cudaMemcpyDeviceToHost, r->m->stream), "radar moments"));
-  return cuda_status(cudaStreamSynchronize(r->m->stream), "radar moments");
+  return cuda_status(copy_to_host(host, r->d_mom, need * sizeof(float), r->m->stream), "radar moments");
 }
 
 int ob_radar_write(ObRadar* r, const void* host, size_t bytes) {
@@ -1825,9 +1824,9 @@ int ob_radar_level2(ObRadar* r, const ObL2Sweep* sweeps, int nsweeps, const uint
   if (rc == OB_OK) {
     launch_level2(r->d_out, r->bytes, static_cast<const ObL2Sweep*>(d_sw), nsweeps, max_nrad, static_cast<const uint8_t*>(d_tpl),
                   static_cast<uint8_t*>(d_o), st);
-    rc = cuda_status(cudaMemcpyAsync(host_out, d_o, out_bytes, cudaMemcpyDeviceToHost, st), "level2 readback");
+    rc = cuda_status(cudaGetLastError(), "level2 launch");
   }
-  if (rc == OB_OK) rc = cuda_status(cudaStreamSynchronize(st), "level2");
+  if (rc == OB_OK) rc = cuda_status(copy_to_host(host_out, d_o, out_bytes, st), "level2 readback");
   for (void* p : {d_sw, d_tpl, d_o})
     if (p) cudaFree(p);
   return rc;
@@ -1835,8 +1834,7 @@ int ob_radar_level2(ObRadar* r, const ObL2Sweep* sweeps, int nsweeps, const uint
 
 int ob_radar_read(ObRadar* r, void* host, size_t bytes) {
   if (!r || !host || bytes > r->bytes) { set_error("ob_radar_read: bad arguments"); return OB_ERR_INVALID; }
-  OB_TRY(cuda_status(cudaMemcpyAsync(host, r->d_out, bytes, cudaMemcpyDeviceToHost, r->m->stream), "radar read"));
-  return cuda_status(cudaStreamSynchronize(r->m->stream), "radar read");
+  return cuda_status(copy_to_host(host, r->d_out, bytes, r->m->stream), "radar read");
 }
 
 int ob_radar_kdp(ObRadar* r, float* host, size_t count) {
