@@ -1245,11 +1245,20 @@ __global__ void k_rain_grp(const uint2* __restrict__ map, int par) {
 // ---------------------------------------------------------------------------------------------------------------
 // WGSL_M_MAP (model.js:1028-1100): 16 diagnostics per column
 // ---------------------------------------------------------------------------------------------------------------
-__global__ void k_maps(Grid g, Uni U, Fields F, float4* out) {
+// A block takes 32 columns of a row (one brick wide); its eight warps share the levels, kMapLevels at a time. What needs
+// an order (the updraft-helicity sum upwards, the cloud-top radiance downwards) leaves its terms in shared memory for
+// the first warp to add in that order; the maxima need none. Levels whose brick holds no precipitation have -30 dBZ and
+// levels without any hydrometeor are transparent (F.actQ0). One thread per column spent its time
+// on the latency of nz levels in turn: 72 -> 22 us at 64 x 64 x 40, 74 -> 33 us at 203 x 157 x 40; from 320 x 320 on, where
+// there are threads enough either way, 112 -> 96 us at 56 levels and no change at 640 x 640 (0.25 ms).
+constexpr int kMapWarps = 8, kMapLevels = 32;
+__global__ void __launch_bounds__(32 * kMapWarps) k_maps(Grid g, Uni U, Fields F, float4* out) {
   constexpr int par = 0;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= g.nx || j >= g.ny) return;
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
+  __shared__ float s_uh[kMapLevels][32], s_a[kMapLevels][32], s_t[kMapLevels][32];
+  __shared__ float s_max[2][kMapWarps][32];
+  const int bx = int(blockIdx.x % unsigned(F.nbx)), j = int(blockIdx.x / unsigned(F.nbx)), lane = threadIdx.x, warp = threadIdx.y;
+  const int nx = g.nx, ny = g.ny, nz = g.nz, i = bx * 32 + lane;
+  const bool in = i < nx;
   const float* const* V = F.V[par];
   auto L = [&](int ch, int a, int b, int c) { return __ldg(V[ch] + g.at(clampi(a, 0, nx), clampi(b, 0, ny), clampi(c, 0, nz))); };
   auto cvel = [&](int a, int b, int c, float v[3]) {
@@ -1258,7 +1267,9 @@ __global__ void k_maps(Grid g, Uni U, Fields F, float4* out) {
     v[2] = 0.5f * (L(2, a, b, c) + L(2, a, b, c + 1));
   };
   const Fall fl{U.step.z, U.micro2.z > 0.5f, U.hur3.w > 0.5f && U.micro2.z <= 0.5f};
+  auto held = [&](int k) { return __ldg(F.actQ0 + bx + F.nbx * ((j >> 2) + F.nby * k)); };
   auto dbz = [&](int k) {
+    if (!(held(k) & 0x38u)) return -30.f;   // no rain, snow or graupel
     const int o = g.at(i, j, k);
     const float rho = bsA(F.B, nz, k).z;
     const float T = __ldg(V[3] + o) * bsB(F.B, nz, k).x;
@@ -1279,13 +1290,59 @@ __global__ void k_maps(Grid g, Uni U, Fields F, float4* out) {
   const float dz = U.dzv.x;
   float comp = -30.f, wmx = 0.f, uh = 0.f;
   const int k12 = min(int(12000.f / dz), nz - 1);
-  for (int k = 0; k < k12; k++) {
-    float v[3];
-    cvel(i, j, k, v);
-    wmx = fmaxf(wmx, v[2]);
-    comp = fmaxf(comp, dbz(k));
-    const float z = (float(k) + 0.5f) * dz;
-    if (z > 2000.f && z < 5000.f && v[2] > 0.f) uh += v[2] * fmaxf(zeta(k), 0.f) * dz;
+  for (int k0 = 0; k0 < k12; k0 += kMapLevels) {
+    const int n = min(kMapLevels, k12 - k0);
+    for (int t = warp; t < n; t += kMapWarps) {
+      const int k = k0 + t;
+      float term = 0.f;
+      if (in) {
+        const float w = 0.5f * (L(2, i, j, k) + L(2, i, j, k + 1));
+        wmx = fmaxf(wmx, w);
+        comp = fmaxf(comp, dbz(k));
+        const float z = (float(k) + 0.5f) * dz;
+        if (z > 2000.f && z < 5000.f && w > 0.f) term = w * fmaxf(zeta(k), 0.f) * dz;
+      }
+      s_uh[t][lane] = term;
+    }
+    __syncthreads();
+    if (warp == 0)
+      for (int t = 0; t < n; t++) uh += s_uh[t][lane];
+    __syncthreads();
+  }
+  s_max[0][warp][lane] = comp;
+  s_max[1][warp][lane] = wmx;
+  // radiance of the column from the top down: opacity and temperature of each level, then the sum in order
+  float tr = 1.f, bt = 0.f;
+  for (int k0 = nz - 1; k0 >= 0; k0 -= kMapLevels) {
+    const int n = min(kMapLevels, k0 + 1);
+    for (int t = warp; t < n; t += kMapWarps) {
+      const int k = k0 - t;
+      float a = 0.f, T = 0.f;
+      if (in) T = __ldg(V[3] + g.at(i, j, k));
+      if (in && (held(k) & 0x3eu)) {
+        const int o = g.at(i, j, k);
+        const float dtau = (80.f * __ldg(F.Q[0][1] + o) + 60.f * __ldg(F.Q[0][2] + o) + 25.f * __ldg(F.Q[0][4] + o) + 4.f * __ldg(F.Q[0][5] + o) +
+                            1.f * __ldg(F.Q[0][3] + o)) * bsA(F.B, nz, k).z * dz;
+        a = 1.f - expf(-dtau);
+      }
+      s_a[t][lane] = a;
+      s_t[t][lane] = T;
+    }
+    __syncthreads();
+    if (warp == 0 && tr >= 1e-3f)
+      for (int t = 0; t < n; t++) {
+        const float a = s_a[t][lane];
+        bt += tr * a * s_t[t][lane] * bsB(F.B, nz, k0 - t).x;
+        tr *= 1.f - a;
+        if (tr < 1e-3f) break;
+      }
+    __syncthreads();
+  }
+  if (warp != 0 || !in) return;
+#pragma unroll
+  for (int w = 1; w < kMapWarps; w++) {
+    comp = fmaxf(comp, s_max[0][w][lane]);
+    wmx = fmaxf(wmx, s_max[1][w][lane]);
   }
   const int k1 = clampi(int(1000.f / dz), 1, nz - 2);
   float v0[3], v1[3];
@@ -1296,16 +1353,6 @@ __global__ void k_maps(Grid g, Uni U, Fields F, float4* out) {
   out[idx] = make_float4(comp, dbz(k1), L(3, i, j, 0) - bsA(F.B, nz, 0).x, zeta(k1));
   out[idx + n2] = make_float4(wmx, uh, conv, sqrtf(v0[0] * v0[0] + v0[1] * v0[1]));
   out[idx + 2 * n2] = make_float4(v0[0], v0[1], v1[0], v1[1]);
-  float tr = 1.f, bt = 0.f;
-  for (int k = nz - 1; k >= 0; k--) {
-    const int o = g.at(i, j, k);
-    const float dtau = (80.f * __ldg(F.Q[0][1] + o) + 60.f * __ldg(F.Q[0][2] + o) + 25.f * __ldg(F.Q[0][4] + o) + 4.f * __ldg(F.Q[0][5] + o) +
-                        1.f * __ldg(F.Q[0][3] + o)) * bsA(F.B, nz, k).z * dz;
-    const float a = 1.f - expf(-dtau);
-    bt += tr * a * __ldg(V[3] + o) * bsB(F.B, nz, k).x;
-    tr *= 1.f - a;
-    if (tr < 1e-3f) break;
-  }
   const float sst = F.sfc[idx].y;
   bt += tr * (sst > 200.f ? sst : L(3, i, j, 0) * bsB(F.B, nz, 0).x);
   const float ps = bsA(F.B, nz, 0).z * U.cn.z * __ldg(F.phi + (i + g.pad) + g.nxp * (j + g.pad)) / 100.f;
@@ -1627,7 +1674,7 @@ void launch_rain(const Grid& g, const Uni& U, const Fields& F, cudaStream_t s) {
   k_rain<<<grid3(g.nx, g.ny, 1, kB2), kB2, 0, s>>>(g, U, F);
 }
 void launch_maps(const Grid& g, const Uni& U, const Fields& F, int par, float4* out, cudaStream_t s) {
-  k_maps<<<grid3(g.nx, g.ny, 1, kB2), kB2, 0, s>>>(g, U, facing(F, par), out);
+  k_maps<<<unsigned(F.nbx) * unsigned(g.ny), dim3(32, kMapWarps), 0, s>>>(g, U, facing(F, par), out);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
