@@ -179,6 +179,8 @@ __device__ __forceinline__ void dst_tc_run(const Src& src, unsigned int* err) {
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  tc::grid_wait();
+  tc::grid_release();
 
   if (warp == 0) {
     if (lane == 0) {  // TMA producer
@@ -458,6 +460,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc::cluster_sync();  // both CTAs' barriers exist before a load or an arrival crosses the pair
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  tc::grid_wait();     // all of the above runs under the tail of the kernel before
+  tc::grid_release();
 
   if (warp == 0) {
     if (lane == 0) {  // TMA producer of this CTA's half of every stage
@@ -612,6 +616,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 __global__ void k_split_rows(const float* __restrict__ src, long rows, int cols, __nv_bfloat16* __restrict__ hi,
                              __nv_bfloat16* __restrict__ lo, int ld) {
+  tc::grid_wait();
+  tc::grid_release();
   const long n = rows * ld;
   for (long t = blockIdx.x * long(blockDim.x) + threadIdx.x; t < n; t += long(gridDim.x) * blockDim.x) {
     const long r = t / ld;
@@ -645,6 +651,7 @@ __device__ __forceinline__ void resid_body(int nx, int ny, int nz, double idx2, 
 }
 __global__ void k_resid(int nx, int ny, int nz, double idx2, const float4* __restrict__ zop, const float* __restrict__ rhs,
                         const float* __restrict__ phi, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int ld) {
+  tc::grid_wait();   // no grid_release: from 1e5 blocks of four warps it doubles the kernel's time; the next kernel starts as they end
   resid_body(nx, ny, nz, idx2, zop, rhs, phi, hi, lo, ld, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 // FP64 norms of the residual r = rhs - A phi (A as in resid_body) and of rhs, over a grid-stride loop: each block
@@ -780,6 +787,8 @@ __device__ __forceinline__ void tri_tma_tile(const CUtensorMap* tIn, const CUten
     tc::fence_mbar_init();
   }
   __syncthreads();
+  tc::grid_wait();
+  tc::grid_release();
   if (tid == 0) {
     tc::mbar_expect_tx(bar, NZ * TRI_TM * TRI_TL * 4);
     tc::tma_load_3d(tile, tIn, bar, l0, m0, 0);
@@ -1035,6 +1044,13 @@ static void set_smem_attrs() {
 
 static inline long pad8(long n) { return (n + 7) / 8 * 8; }
 
+// Standalone solves of at most this many cells, and every solve of a model's step, launch their kernels early
+// (launch_early): in one stream that is always faster, 116 -> 89 us at 80 x 80 x 40, 250 -> 221 us at 336 x 336 x 40, 673 ->
+// 658 us at 656 x 656 x 40. But a block that waits holds its SM's shared memory, which other streams' kernels then cannot
+// have: three handles solving at once take 46 -> 38 us a solve at 80 x 80 x 40, 101 us either way at 240 x 240 x 40 (2.3e6
+// cells) and 168 -> 183 us at 300 x 300 x 40. A model's solve has its step's side streams idle.
+constexpr long kEarlyCells = 1l << 21;
+
 struct TcPlan {
   int nx, ny, nz;
   long ldx, ldy;
@@ -1057,6 +1073,7 @@ struct TcPlan {
   long ld2 = 0;          // row pitch of T2 (floats, whole 16 bytes: the tensor map's rule)
   float4 zh[80] = {};    // the z-operator on the host: the by-value coefficients of k_tri_tma (nz <= 80)
   CUtensorMap Qh[4][2];  // the DST matrices with boxes of half a tile's width: each CTA of a pair loads one half
+  bool early = false;    // kernels set themselves up under the tail of the one before (launch_early)
   bool pairs = true;     // transforms on SM pairs (k_dst_tc2); single-SM tiles (k_dst_tc) when false
 };
 
@@ -1202,7 +1219,24 @@ void PoissonPlan::tc_destroy() {
   tc = nullptr;
 }
 
-static cudaLaunchConfig_t pair_config(int pairs, cudaStream_t s, cudaLaunchAttribute* at) {
+// a launch whose kernel, if early, sets itself up (barriers, TMEM, tensor maps) under the tail of the kernel before it in
+// the stream (tc::grid_wait)
+template <class... P, class... A>
+static void launch_early(bool early, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
+static cudaLaunchConfig_t pair_config(bool early, int pairs, cudaStream_t s, cudaLaunchAttribute* at) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(kThreads);
@@ -1212,8 +1246,10 @@ static cudaLaunchConfig_t pair_config(int pairs, cudaStream_t s, cudaLaunchAttri
   at[0].val.clusterDim.x = 2;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_early
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 2 : 1;
   return cfg;
 }
 
@@ -1222,8 +1258,8 @@ static cudaLaunchConfig_t pair_config(int pairs, cudaStream_t s, cudaLaunchAttri
 static int pair_slots() {
   static int n = 0;
   if (!n) {
-    cudaLaunchAttribute at[1];
-    const cudaLaunchConfig_t cfg = pair_config(num_sms() / 2, nullptr, at);
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = pair_config(false, num_sms() / 2, nullptr, at);
     if (cudaOccupancyMaxActiveClusters(&n, k_dst_tc2<OUT_T_F32>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = num_sms() / 2;
@@ -1263,18 +1299,18 @@ static PairSched pair_sched(int M, int N, int BN, int max_pairs, int& pairs) {
 }
 
 template <int MODE, bool ONE = false>
-static void launch_tc(const CUtensorMap* f, const CUtensorMap* q, int K, int bn, const TcOut& o, unsigned int* err, cudaStream_t s,
+static void launch_tc(bool early, const CUtensorMap* f, const CUtensorMap* q, int K, int bn, const TcOut& o, unsigned int* err, cudaStream_t s,
                       const CUtensorMap* qh = nullptr) {
   if (qh) {  // SM pairs: tiles of 256 field rows, qh the DST matrix maps with half-width boxes
     int pairs = 0;
     const PairSched sc = pair_sched(o.M, o.N, bn, pair_slots(), pairs);
-    cudaLaunchAttribute at[1];
-    const cudaLaunchConfig_t cfg = pair_config(pairs, s, at);
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = pair_config(early, pairs, s, at);
     cudaLaunchKernelEx(&cfg, k_dst_tc2<MODE, ONE>, f[0], f[1], qh[0], qh[1], K, sc, o, err);
     return;
   }
   const int tiles = ((o.M + BM - 1) / BM) * ((o.N + bn - 1) / bn);
-  k_dst_tc<MODE, ONE><<<std::min(tiles, num_sms()), kThreads, SMEM_BYTES, s>>>(f[0], f[1], q[0], q[1], K, bn, o, err);
+  launch_early(early, k_dst_tc<MODE, ONE>, std::min(tiles, num_sms()), kThreads, SMEM_BYTES, s, f[0], f[1], q[0], q[1], K, bn, o, err);
 }
 
 // the TMA tridiagonals of one pass: the z-operator goes by value (the host copy of set_density's coefficients)
@@ -1283,8 +1319,8 @@ static void launch_tri_tma(const TcPlan* T, const float* lam, bool hi_only, cuda
   TriZ<NZ> Z;
   for (int k = 0; k < NZ; k++) Z.z[k] = T->zh[k];
   const dim3 grid((T->nx + TRI_TL - 1) / TRI_TL, (T->ny + TRI_TM - 1) / TRI_TM);
-  if (hi_only) k_tri_tma<NZ, true><<<grid, TRI_TL * TRI_TM, tri_smem_bytes<NZ>(), s>>>(T->tri_in, T->tri_out[0], T->tri_out[1], T->nx, T->ny, lam, Z, T->low, T->err);
-  else k_tri_tma<NZ, false><<<grid, TRI_TL * TRI_TM, tri_smem_bytes<NZ>(), s>>>(T->tri_in, T->tri_out[0], T->tri_out[1], T->nx, T->ny, lam, Z, T->low, T->err);
+  launch_early(T->early, hi_only ? k_tri_tma<NZ, true> : k_tri_tma<NZ, false>, grid, TRI_TL * TRI_TM, tri_smem_bytes<NZ>(), s, T->tri_in, T->tri_out[0],
+               T->tri_out[1], T->nx, T->ny, lam, Z, T->low, T->err);
 }
 
 // the four transforms and the tridiagonals from a split right-hand side (rx, or the residual rr when add) to phi
@@ -1295,11 +1331,11 @@ static void tc_pass(const PoissonPlan& P, TcPlan* T, const float* lam, float* ph
   const int nx = P.nx, ny = P.ny, nz = P.nz;
   const TcOut sy{T->sy_hi, T->sy_lo, nullptr, T->ldy, ny, nz * ny, nx}, t2{nullptr, nullptr, T->t2, T->ld2, nx, nz * nx, ny};
   // X-fwd: field rows (k, j), K = i, outputs l  -> S_y[k][l][j]
-  if (one) launch_tc<OUT_T_BF16X2, true>(add ? T->Frr : T->Fr, T->Q[0], nx, T->bnx, sy, T->err, s, QH(0));
-  else launch_tc<OUT_T_BF16X2>(add ? T->Frr : T->Fr, T->Q[0], nx, T->bnx, sy, T->err, s, QH(0));
+  if (one) launch_tc<OUT_T_BF16X2, true>(T->early, add ? T->Frr : T->Fr, T->Q[0], nx, T->bnx, sy, T->err, s, QH(0));
+  else launch_tc<OUT_T_BF16X2>(T->early, add ? T->Frr : T->Fr, T->Q[0], nx, T->bnx, sy, T->err, s, QH(0));
   // Y-fwd: field rows (k, l), K = j, outputs m  -> T2[k][m][l] fp32
-  if (one) launch_tc<OUT_T_F32, true>(T->Fy, T->Q[1], ny, T->bny, t2, T->err, s, QH(1));
-  else launch_tc<OUT_T_F32>(T->Fy, T->Q[1], ny, T->bny, t2, T->err, s, QH(1));
+  if (one) launch_tc<OUT_T_F32, true>(T->early, T->Fy, T->Q[1], ny, T->bny, t2, T->err, s, QH(1));
+  else launch_tc<OUT_T_F32>(T->early, T->Fy, T->Q[1], ny, T->bny, t2, T->err, s, QH(1));
   // tridiagonals -> S_y[k][l][m]
   // (a plain-bf16 pass writes the hi plane alone: its y-inverse transform reads nothing else)
   switch (nz) {
@@ -1309,14 +1345,14 @@ static void tc_pass(const PoissonPlan& P, TcPlan* T, const float* lam, float* ph
   }
   // Y-inv: field rows (k, l), K = m, outputs j  -> S_x[k][j][l]
   const TcOut sx{T->sx_hi, T->sx_lo, nullptr, T->ldx, nx, nz * nx, ny};
-  if (one) launch_tc<OUT_T_BF16X2, true>(T->Fy, T->Q[2], ny, T->bny, sx, T->err, s, QH(2));
-  else launch_tc<OUT_T_BF16X2>(T->Fy, T->Q[2], ny, T->bny, sx, T->err, s, QH(2));
+  if (one) launch_tc<OUT_T_BF16X2, true>(T->early, T->Fy, T->Q[2], ny, T->bny, sx, T->err, s, QH(2));
+  else launch_tc<OUT_T_BF16X2>(T->early, T->Fy, T->Q[2], ny, T->bny, sx, T->err, s, QH(2));
   // X-inv: field rows (k, j), K = l, outputs i  -> phi[k][j][i]
   const TcOut o{nullptr, nullptr, phi, nx, ny, nz * ny, nx};
-  if (one && add) launch_tc<OUT_R_F32_ADD, true>(T->Fx, T->Q[3], nx, T->bnx, o, T->err, s, QH(3));
-  else if (one) launch_tc<OUT_R_F32, true>(T->Fx, T->Q[3], nx, T->bnx, o, T->err, s, QH(3));
-  else if (add) launch_tc<OUT_R_F32_ADD>(T->Fx, T->Q[3], nx, T->bnx, o, T->err, s, QH(3));
-  else launch_tc<OUT_R_F32>(T->Fx, T->Q[3], nx, T->bnx, o, T->err, s, QH(3));
+  if (one && add) launch_tc<OUT_R_F32_ADD, true>(T->early, T->Fx, T->Q[3], nx, T->bnx, o, T->err, s, QH(3));
+  else if (one) launch_tc<OUT_R_F32, true>(T->early, T->Fx, T->Q[3], nx, T->bnx, o, T->err, s, QH(3));
+  else if (add) launch_tc<OUT_R_F32_ADD>(T->early, T->Fx, T->Q[3], nx, T->bnx, o, T->err, s, QH(3));
+  else launch_tc<OUT_R_F32>(T->early, T->Fx, T->Q[3], nx, T->bnx, o, T->err, s, QH(3));
 #undef QH
 }
 
@@ -1333,12 +1369,13 @@ int PoissonPlan::tc_solve(const float* rhs, float* phi, cudaStream_t s) {
   if (!presplit || precision >= 2) {
     if (!rhs) { set_error("poisson: right-hand side missing"); return OB_ERR_INVALID; }
   }
-  if (!presplit) k_split_rows<<<1184, 256, 0, s>>>(rhs, long(nz) * ny, nx, T->rx_hi, T->rx_lo, int(T->ldx));
+  T->early = presplit || long(nx) * ny * nz <= kEarlyCells;
+  if (!presplit) launch_early(T->early, k_split_rows, 1184, 256, 0, s, rhs, long(nz) * ny, nx, T->rx_hi, T->rx_lo, int(T->ldx));
   tc_pass(*this, T, lam, phi, false, s, precision == 5);
   if (precision >= 2) {
     const int sweeps = precision == 4 ? 2 : 1;
     for (int sw = 0; sw < sweeps; sw++) {
-      k_resid<<<dim3((nx + 127) / 128, ny, nz), 128, 0, s>>>(nx, ny, nz, 1.0 / (dx * dx), zop, rhs, phi, T->rr_hi, T->rr_lo, int(T->ldx));
+      launch_early(T->early, k_resid, dim3((nx + 127) / 128, ny, nz), 128, 0, s, nx, ny, nz, 1.0 / (dx * dx), zop, rhs, phi, T->rr_hi, T->rr_lo, int(T->ldx));
       tc_pass(*this, T, lam, phi, true, s, precision == 3);
     }
   }
@@ -1663,7 +1700,7 @@ extern "C" int ob_dst_tc_selftest(int M, int N, int K, int planes, const float* 
   if (rc == OB_OK) {
     set_smem_attrs();
     const TcOut o{nullptr, nullptr, dc, N, N, planes * N, M};  // C[p][m][n] = out[(p * M + m) * N + n]
-    launch_tc<OUT_T_F32>(tf, tq, K, bn, o, derr, nullptr);
+    launch_tc<OUT_T_F32>(false, tf, tq, K, bn, o, derr, nullptr);
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) { set_error("ob_dst_tc_selftest: %s", cudaGetErrorString(e)); rc = OB_ERR_DEVICE; }
     unsigned int h = 0;

@@ -43,6 +43,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
   return false;
 }
 
+// Programmatic dependent launch: a kernel launched with that attribute may start while the kernel before it in the stream
+// still runs. grid_wait returns once that kernel has completed and its writes are visible (at once when there is none);
+// every thread calls it before its first access to memory that other kernels write or read. grid_release lets the next
+// kernel start setting itself up when all blocks have called it or left.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // TMA tile loads (no multicast)
 __device__ __forceinline__ void tma_load_2d(void* smem, const void* tmap, uint64_t* bar, int c0, int c1) {
   asm volatile(
