@@ -1219,23 +1219,6 @@ void PoissonPlan::tc_destroy() {
   tc = nullptr;
 }
 
-// a launch whose kernel, if early, sets itself up (barriers, TMEM, tensor maps) under the tail of the kernel before it in
-// the stream (tc::grid_wait)
-template <class... P, class... A>
-static void launch_early(bool early, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = at;
-  cfg.numAttrs = early ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
-}
-
 static cudaLaunchConfig_t pair_config(bool early, int pairs, cudaStream_t s, cudaLaunchAttribute* at) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
@@ -1310,7 +1293,7 @@ static void launch_tc(bool early, const CUtensorMap* f, const CUtensorMap* q, in
     return;
   }
   const int tiles = ((o.M + BM - 1) / BM) * ((o.N + bn - 1) / bn);
-  launch_early(early, k_dst_tc<MODE, ONE>, std::min(tiles, num_sms()), kThreads, SMEM_BYTES, s, f[0], f[1], q[0], q[1], K, bn, o, err);
+  tc::launch_early(early, k_dst_tc<MODE, ONE>, std::min(tiles, num_sms()), kThreads, SMEM_BYTES, s, f[0], f[1], q[0], q[1], K, bn, o, err);
 }
 
 // the TMA tridiagonals of one pass: the z-operator goes by value (the host copy of set_density's coefficients)
@@ -1319,7 +1302,7 @@ static void launch_tri_tma(const TcPlan* T, const float* lam, bool hi_only, cuda
   TriZ<NZ> Z;
   for (int k = 0; k < NZ; k++) Z.z[k] = T->zh[k];
   const dim3 grid((T->nx + TRI_TL - 1) / TRI_TL, (T->ny + TRI_TM - 1) / TRI_TM);
-  launch_early(T->early, hi_only ? k_tri_tma<NZ, true> : k_tri_tma<NZ, false>, grid, TRI_TL * TRI_TM, tri_smem_bytes<NZ>(), s, T->tri_in, T->tri_out[0],
+  tc::launch_early(T->early, hi_only ? k_tri_tma<NZ, true> : k_tri_tma<NZ, false>, grid, TRI_TL * TRI_TM, tri_smem_bytes<NZ>(), s, T->tri_in, T->tri_out[0],
                T->tri_out[1], T->nx, T->ny, lam, Z, T->low, T->err);
 }
 
@@ -1370,12 +1353,12 @@ int PoissonPlan::tc_solve(const float* rhs, float* phi, cudaStream_t s) {
     if (!rhs) { set_error("poisson: right-hand side missing"); return OB_ERR_INVALID; }
   }
   T->early = presplit || long(nx) * ny * nz <= kEarlyCells;
-  if (!presplit) launch_early(T->early, k_split_rows, 1184, 256, 0, s, rhs, long(nz) * ny, nx, T->rx_hi, T->rx_lo, int(T->ldx));
+  if (!presplit) tc::launch_early(T->early, k_split_rows, 1184, 256, 0, s, rhs, long(nz) * ny, nx, T->rx_hi, T->rx_lo, int(T->ldx));
   tc_pass(*this, T, lam, phi, false, s, precision == 5);
   if (precision >= 2) {
     const int sweeps = precision == 4 ? 2 : 1;
     for (int sw = 0; sw < sweeps; sw++) {
-      launch_early(T->early, k_resid, dim3((nx + 127) / 128, ny, nz), 128, 0, s, nx, ny, nz, 1.0 / (dx * dx), zop, rhs, phi, T->rr_hi, T->rr_lo, int(T->ldx));
+      tc::launch_early(T->early, k_resid, dim3((nx + 127) / 128, ny, nz), 128, 0, s, nx, ny, nz, 1.0 / (dx * dx), zop, rhs, phi, T->rr_hi, T->rr_lo, int(T->ldx));
       tc_pass(*this, T, lam, phi, true, s, precision == 3);
     }
   }
