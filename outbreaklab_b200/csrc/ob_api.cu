@@ -446,6 +446,7 @@ int ob_model_create(const ObGrid* grid, ObModel** out) {
   m->F.bnd = m->d_bnd;
   m->F.ci = m->d_ci;
   m->F.flags = m->d_flags;
+  m->F.vmax = m->d_flags + 8;
   m->F.clock = m->d_clock;
   m->F.nbx = nbx;
   m->F.nby = nby;
@@ -631,6 +632,7 @@ static int enqueue_step(ObModel* m, bool lsf, cudaStream_t s) {
     const size_t bytes = m->fs * sizeof(float);
     for (int c = 0; c < 4; c++) OB_TRY(cuda_status(cudaMemcpyAsync(m->F.V[par][c], m->F.V[1 - par][c], bytes, cudaMemcpyDeviceToDevice, s), "filter"));
     for (int c = 0; c < 8; c++) OB_TRY(cuda_status(cudaMemcpyAsync(m->F.Q[0][c], m->F.Q[1][c], bytes, cudaMemcpyDeviceToDevice, s), "filter"));
+    launch_activity(g, m->F, s);   // the filter spreads the scalars past the bricks that held them
   }
   if (m->hur_on) launch_prep(g, m->U, m->F, par, s);
   if (lsf) launch_lsf(g, m->U, m->F, s);
@@ -910,6 +912,7 @@ int ob_model_profile_step(ObModel* m, float dt, float* ms, int max_passes) {
   cudaEventRecord(ev[e++], s);
   launch_advv(g, m->U, m->F, par, s);
   cudaEventRecord(ev[e++], s);
+  if (m->hur_on) cudaMemsetAsync(m->F.vmax, 0x7f, 3 * sizeof(unsigned), s);   // no prep pass here to bound the winds
   launch_advq(g, m->U, m->F, par, s);
   cudaEventRecord(ev[e++], s);
   const int prc = physics_pass(m, par, s);

@@ -58,6 +58,7 @@ struct Fields {
   const float* bnd; // OB_MAX_BOUNDS x 148
   const float* ci;  // events x 12
   unsigned int* flags;  // [0] NaN/Inf counter
+  unsigned int* vmax;   // hurricane mode: bits of the step's largest |u|, |v|, |w|
   // skip of absent hydrometeor and spare channels, per brick of 32 x 4 x 1 cells (nbx x nby x nz bricks): bit c of a
   // flag word stands for channel c (1..7)
   unsigned int* actQ0;   // Q slot 0 may hold the channel in the brick

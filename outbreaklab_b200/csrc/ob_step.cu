@@ -430,20 +430,6 @@ __global__ void k_advv1_grp(const uint2* __restrict__ map, int par) {
   advv1_body(c_members[mem].g, c_members[mem].U, c_members[mem].F, par, gbx, gby, gbz);
 }
 
-__device__ __forceinline__ float2 minmax8V(const float* __restrict__ f, const Grid& g, float x, float y, float z, float ox, float oy, float oz) {
-  // the trace is clamped to the box, so each floor index lies in [-1, n] and one bound per corner clamps it
-  const int i0 = __float2int_rd(x - ox), j0 = __float2int_rd(y - oy), k0 = __float2int_rd(z - oz);
-  const int ia = max(i0, 0), ib = min(i0 + 1, g.nx), ja = max(j0, 0), jb = min(j0 + 1, g.ny), ka = max(k0, 0), kb = min(k0 + 1, g.nz);
-  float lo = 1e30f, hi = -1e30f;
-#pragma unroll
-  for (int q = 0; q < 8; q++) {
-    const float s = __ldg(f + g.at((q & 1) ? ib : ia, ((q >> 1) & 1) ? jb : ja, (q >> 2) ? kb : ka));
-    lo = fminf(lo, s);
-    hi = fmaxf(hi, s);
-  }
-  return make_float2(lo, hi);
-}
-
 __device__ __forceinline__ void advv2_body(const Grid& g, const Uni& U, const Fields& F, int par, const int BX, const int BY, const int BZ) {
   OB_TEXEL_LOOP_BEGIN(g.nx, g.ny, g.nz)
   const Loc L = localVel(F, g, par, ci, cj, ck);
@@ -538,7 +524,29 @@ __device__ __forceinline__ unsigned block_or(unsigned v) {
 struct Region {
   int x0, x1, y0, y1, z0, z1;
 };
-// the channels that a brick touching the block's region holds (bits 1..7), the same for all threads of the block
+// the channels (bits 1..7) that the bricks of a box of cells hold, in every thread of the block; the caller has set held
+// to 0 and synchronised since
+__device__ __forceinline__ unsigned box_channels(const Grid& g, const Fields& F, Region r, const unsigned int* flagsA,
+                                                 const unsigned int* flagsB, unsigned& held) {
+  const int bx0 = clampi(r.x0, 0, g.nx - 1) / 32, bx1 = clampi(r.x1, 0, g.nx - 1) / 32;
+  const int by0 = clampi(r.y0, 0, g.ny - 1) / 4, by1 = clampi(r.y1, 0, g.ny - 1) / 4;
+  const int bz0 = clampi(r.z0, 0, g.nz - 1), bz1 = clampi(r.z1, 0, g.nz - 1);
+  const int nxb = bx1 - bx0 + 1, nyb = by1 - by0 + 1, nzb = bz1 - bz0 + 1;
+  const int count = nxb * nyb * nzb;
+  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+  unsigned any = 0;
+  for (int t = tid; t < count; t += blockDim.x * blockDim.y) {
+    const int bx = bx0 + t % nxb, by = by0 + (t / nxb) % nyb, bz = bz0 + t / (nxb * nyb);
+    const int b = bx + F.nbx * (by + F.nby * bz);
+    any |= __ldg(flagsA + b);
+    if (flagsB) any |= __ldg(flagsB + b);
+  }
+  any = __reduce_or_sync(0xffffffffu, any);
+  if ((threadIdx.x & 31) == 0 && any) atomicOr(&held, any);
+  __syncthreads();
+  return held;
+}
+// the channels that a brick touching the block's region holds, the region spanned by its threads' boxes r
 __device__ __forceinline__ unsigned region_channels(const Grid& g, const Fields& F, Region r, const unsigned int* flagsA,
                                                     const unsigned int* flagsB) {
   __shared__ int red[6];
@@ -560,23 +568,7 @@ __device__ __forceinline__ unsigned region_channels(const Grid& g, const Fields&
     atomicMin(&red[4], c0); atomicMax(&red[5], c1);
   }
   __syncthreads();
-  const int bx0 = clampi(red[0], 0, g.nx - 1) / 32, bx1 = clampi(red[1], 0, g.nx - 1) / 32;
-  const int by0 = clampi(red[2], 0, g.ny - 1) / 4, by1 = clampi(red[3], 0, g.ny - 1) / 4;
-  const int bz0 = clampi(red[4], 0, g.nz - 1), bz1 = clampi(red[5], 0, g.nz - 1);
-  const int nxb = bx1 - bx0 + 1, nyb = by1 - by0 + 1, nzb = bz1 - bz0 + 1;
-  const int count = nxb * nyb * nzb;
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-  unsigned any = 0;
-  for (int t = tid; t < count; t += blockDim.x * blockDim.y) {
-    const int bx = bx0 + t % nxb, by = by0 + (t / nxb) % nyb, bz = bz0 + t / (nxb * nyb);
-    const int b = bx + F.nbx * (by + F.nby * bz);
-    any |= __ldg(flagsA + b);
-    if (flagsB) any |= __ldg(flagsB + b);
-  }
-  any = __reduce_or_sync(m, any);
-  if ((threadIdx.x & 31) == 0 && any) atomicOr(&held, any);
-  __syncthreads();
-  return held;
+  return box_channels(g, F, Region{red[0], red[1], red[2], red[3], red[4], red[5]}, flagsA, flagsB, held);
 }
 
 // ---- ADVQ1 (model.js:500-529): semi-Lagrangian step of the 8 scalars, channels grouped by the fall speed of
@@ -1155,9 +1147,9 @@ __global__ void __launch_bounds__(128, (MM == kMicroSurrogate && BND == 1) ? 9 :
   constexpr int par = 0;
   phys_body<MM, false, BND>(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z);
 }
+template <int BND>
 __global__ void __launch_bounds__(128) k_phys_hur(Grid g, Uni U, Fields F) {
-  constexpr int par = 0;
-  phys_body<kMicroPlain, true>(g, U, F, par, blockIdx.x, blockIdx.y, blockIdx.z);
+  phys_body<kMicroPlain, true, BND>(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <int MM>
 __global__ void __launch_bounds__(128, 9) k_phys_grp(const uint2* __restrict__ map, int par) {
@@ -1384,8 +1376,7 @@ __global__ void k_unpack(Grid g, Ptr8 dst, int nch, int X, int Y, int Z, const f
 
 // ---------------------------------------------------------------------------------------------------------------
 // hurricane mode: the advection with midpoint trajectories and settling ice, the pressure force carried along the
-// trajectories (WGSL_M_PREP) and the 2-dx filter (WGSL_M_FILT). Straight restatements, one thread per texel, no
-// clear-air skip (these runs are the few, not the bench's).
+// trajectories (WGSL_M_PREP) and the 2-dx filter (WGSL_M_FILT), one thread per texel.
 // ---------------------------------------------------------------------------------------------------------------
 // the winds at a point in grid units, from the true winds (model.js:420-423)
 __device__ __forceinline__ void velAt(const Fields& F, const Grid& g, int par, float x, float y, float z, float v[3]) {
@@ -1440,6 +1431,28 @@ __global__ void k_prep(Grid g, Uni U, Fields F) {
   F.Vp[2][o] = w;
   F.Vp[3][o] = __ldg(F.V[par][3] + o);
 }
+// the domain's largest |u|, |v| and |w| (as the bits of a float, which order as integers; a NaN counts as infinite) into
+// F.vmax, which the host has set to 0: they bound every trajectory of the step
+__global__ void __launch_bounds__(256) k_wind_max(Grid g, Fields F) {
+  __shared__ unsigned red[3];
+  if (threadIdx.x < 3) red[threadIdx.x] = 0u;
+  __syncthreads();
+  const long rows = long(g.ny + 1) * (g.nz + 1);
+  unsigned m[3] = {0u, 0u, 0u};
+  for (long r = long(blockIdx.x) * 8 + (threadIdx.x >> 5); r < rows; r += long(gridDim.x) * 8) {   // a warp per row
+    const long base = r * g.px;
+    for (int i = threadIdx.x & 31; i <= g.nx; i += 32)
+#pragma unroll
+      for (int c = 0; c < 3; c++) m[c] = max(m[c], __float_as_uint(__ldg(F.V[0][c] + base + i)) & 0x7fffffffu);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const unsigned w = __reduce_max_sync(0xffffffffu, m[c]);
+    if ((threadIdx.x & 31) == 0) atomicMax(&red[c], w);
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMax(F.vmax + threadIdx.x, red[threadIdx.x]);
+}
 
 // 4th-order horizontal hyperdiffusion of V and Q into V[1-par], Q slot 1 (model.js:948-994)
 __global__ void k_filt(Grid g, Uni U, Fields F) {
@@ -1466,7 +1479,9 @@ __global__ void k_filt(Grid g, Uni U, Fields F) {
   }
 }
 
-// ADVV1/2 of hurricane mode (model.js:434-481): trajectories from the true winds, values carried from Vp
+// ADVV1/2 of hurricane mode (model.js:434-481): trajectories from the true winds, values carried from Vp. As in the outbreak
+// passes, ADVV1 keeps the limiter's window of its departure sample, so that ADVV2 traces forwards alone (a trajectory
+// costs 24 gathers for its midpoint wind): ADVV2 292 -> 145 us at 256 x 224 x 40.
 __global__ void k_advv1_hur(Grid g, Uni U, Fields F) {
   constexpr int par = 0;
   OB_BLOCKS_DIRECT
@@ -1474,14 +1489,18 @@ __global__ void k_advv1_hur(Grid g, Uni U, Fields F) {
   const Loc L = localVel(F, g, par, ci, cj, ck);
   const float kk[3] = {U.der.x, U.der.x, U.der.y};
   const float fi = float(ci), fj = float(cj), fk = float(ck);
-  const int o = g.at(ci, cj, ck);
+  const unsigned o = 4u * unsigned(g.at(ci, cj, ck));
   const float P[4][3] = {{fi, fj + 0.5f, fk + 0.5f}, {fi + 0.5f, fj, fk + 0.5f}, {fi + 0.5f, fj + 0.5f, fk}, {fi + 0.5f, fj + 0.5f, fk + 0.5f}};
   const float* vel[4] = {L.vu, L.vv, L.vw, L.vc};
 #pragma unroll
   for (int c = 0; c < 4; c++) {
-    float x, y, z;
+    const float ox = c == 0 ? 0.f : 0.5f, oy = c == 1 ? 0.f : 0.5f, oz = c == 2 ? 0.f : 0.5f;
+    float x, y, z, lo, hi;
     traceH(U, F, g, par, kk, P[c][0], P[c][1], P[c][2], vel[c], 1.f, x, y, z);
-    F.Vt[c][o] = sampleVch(F.Vp[c], g, c, x, y, z);
+    const float t = trilerpB_mm(F.Vp[c], g, g.nx + 1, g.ny + 1, g.nz + 1, x - ox, y - oy, z - oz, lo, hi);
+    sto(F.Vt[c], o, t);
+    sto(F.Vlo[c], o, lo);
+    sto(F.Vhi[c], o, hi);
   }
 }
 __global__ void k_advv2_hur(Grid g, Uni U, Fields F) {
@@ -1496,95 +1515,147 @@ __global__ void k_advv2_hur(Grid g, Uni U, Fields F) {
   const float cx = L.vc[0] * kk[0], cy = L.vc[1] * kk[1], cz = L.vc[2] * kk[2];
   const float cour = sqrtf(cx * cx + cy * cy + cz * cz);
   const float sm = 0.5f * U.misc.y * clampf(cour / 0.35f, U.dzv.w, 1.f);
-  const int o = g.at(ci, cj, ck);
+  const unsigned o = 4u * unsigned(g.at(ci, cj, ck));
 #pragma unroll
   for (int c = 0; c < 4; c++) {
-    const float ox = c == 0 ? 0.f : 0.5f, oy = c == 1 ? 0.f : 0.5f, oz = c == 2 ? 0.f : 0.5f;
     float x, y, z;
     traceH(U, F, g, par, kk, P[c][0], P[c][1], P[c][2], vel[c], -1.f, x, y, z);
     const float b = sampleVch(F.Vt[c], g, c, x, y, z);
-    const float hat = __ldg(F.Vt[c] + o), old = __ldg(F.Vp[c] + o);
+    const float hat = ldo(F.Vt[c], o), old = ldo(F.Vp[c], o);
     const float r = hat + sm * (old - b);
-    traceH(U, F, g, par, kk, P[c][0], P[c][1], P[c][2], vel[c], 1.f, x, y, z);
-    const float2 m = minmax8V(F.Vp[c], g, x, y, z, ox, oy, oz);
-    F.V[1 - par][c][o] = clampf(r, m.x, m.y);
+    sto(F.V[1 - par][c], o, clampf(r, ldo(F.Vlo[c], o), ldo(F.Vhi[c], o)));
   }
 }
 
-// ADVQ1/2 of hurricane mode (model.js:500-576): every channel, maritime graupel, settling ice. The brick flags of the
-// clear-air skip are left saying "may hold hydrometeors", so that a later run without the hurricane stays exact.
-__device__ __forceinline__ void brick_flags_all(const Grid& g, const Fields& F, unsigned* a, unsigned* zq, unsigned* z1) {
-  if (threadIdx.x == 0 && threadIdx.y == 0 && int(blockIdx.x) < F.nbx && int(blockIdx.y) < F.nby && int(blockIdx.z) < g.nz) {
-    const int b = blockIdx.x + F.nbx * (blockIdx.y + F.nby * blockIdx.z);
-    if (a) a[b] = kHydro;
-    if (zq) zq[b] = 0u;
-    if (z1) z1[b] = 0u;
-  }
+// ADVQ1/2 of hurricane mode (model.js:500-576): maritime graupel, settling ice. Channels absent from a block's reach are
+// skipped as in the outbreak passes, but the reach comes from the step's largest winds (F.vmax) instead of the block's own
+// departure points, which would need every channel's trajectory first: a trajectory's wind is a mean of winds, so it ends
+// within dt / dx of that bound (and, downwards and upwards, of it plus the largest fall speed). Channels at the air's
+// speed share one trajectory each way. 256 x 224 x 40 with a storm every 60 km: ADVQ1 210 -> 109 us, ADVQ2 589 -> 220 us,
+// and PHYS, which finds dry blocks by the same flags, 222 -> 193 us; the winds' maxima take 10 us.
+__device__ __forceinline__ unsigned reach_channels(const Grid& g, const Uni& U, const Fields& F, const unsigned int* flagsA,
+                                                   const unsigned int* flagsB) {
+  __shared__ unsigned held;
+  if (threadIdx.x == 0 && threadIdx.y == 0) held = 0u;
+  __syncthreads();
+  auto cells = [](float d) { return d < 1e6f ? int(ceilf(d * 1.001f + 0.01f)) : 1 << 24; };   // also for a NaN
+  const int rx = cells(U.der.x * __uint_as_float(__ldg(F.vmax))), ry = cells(U.der.x * __uint_as_float(__ldg(F.vmax + 1)));
+  const int rz = cells(U.der.y * (__uint_as_float(__ldg(F.vmax + 2)) + F.fallmax));
+  const int x = blockIdx.x * 32, y = blockIdx.y * 4, z = blockIdx.z;
+  return box_channels(g, F, Region{x - rx, x + 32 + rx, y - ry, y + 4 + ry, z - rz, z + 1 + rz}, flagsA, flagsB, held);
 }
-__global__ void k_advq1_hur(Grid g, Uni U, Fields F) {
+__global__ void __launch_bounds__(128) k_advq1_hur(Grid g, Uni U, Fields F) {
   constexpr int par = 0;
-  brick_flags_all(g, F, F.actQt, F.zeroQt, nullptr);
   const int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y, ck = blockIdx.z;
+  const int brick = blockIdx.x + F.nbx * (blockIdx.y + F.nby * blockIdx.z);
+  const unsigned zeros = F.zeroQt[brick];   // read by every thread before the barriers, written after them
+  const unsigned act = reach_channels(g, U, F, F.actQ0, nullptr);
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    F.actQt[brick] = act;
+    F.zeroQt[brick] = kHydro & ~act;
+  }
   if (ci >= g.nx || cj >= g.ny || ck >= g.nz) return;
-  const int o = g.at(ci, cj, ck);
+  auto has = [&](int c) { return ((act >> c) & 1u) != 0u; };
+  const unsigned o = 4u * unsigned(g.at(ci, cj, ck));
   const float kk[3] = {U.der.x, U.der.x, U.der.y};
   const float p[3] = {float(ci) + 0.5f, float(cj) + 0.5f, float(ck) + 0.5f};
   float v[3];
   cellVel(F, g, par, ci, cj, ck, v);
-  const float rho = bsA(F.B, g.nz, ck).z;
-  const bool thm = U.micro2.z > 0.5f;
-  const Fall fl{U.step.z, thm, U.hur3.w > 0.5f && !thm};
-  const float2 fv = fl.vtRain(__ldg(F.Q[0][3] + o), __ldg(F.Q[0][6] + o), rho);
-  const float fs = fl.vtS(__ldg(F.Q[0][4] + o), rho), fg = fl.vtGrau(__ldg(F.Q[0][5] + o), rho), fi = vtI(U, __ldg(F.Q[0][2] + o), rho);
   float x, y, z;
-  auto at = [&](float fall, int c) {
-    traceQH(U, F, g, par, kk, p, v, fall, 1.f, x, y, z);
-    return gatherQ(F.Q[0][c], tapQ(g, x, y, z));
-  };
   traceQH(U, F, g, par, kk, p, v, 0.f, 1.f, x, y, z);
   const Tap t0 = tapQ(g, x, y, z);
-  F.Qt[0][o] = gatherQ(F.Q[0][0], t0);
-  F.Qt[1][o] = gatherQ(F.Q[0][1], t0);
-  F.Qt[2][o] = fi > 0.f ? at(fi, 2) : gatherQ(F.Q[0][2], t0);
-  F.Qt[3][o] = at(fv.x, 3);
-  F.Qt[4][o] = at(fs, 4);
-  F.Qt[5][o] = at(fg, 5);
-  F.Qt[6][o] = thm ? at(fv.y, 6) : gatherQ(F.Q[0][6], t0);
-  F.Qt[7][o] = gatherQ(F.Q[0][7], t0);
+  sto(F.Qt[0], o, gatherQ(F.Q[0][0], t0));
+  if (act) {
+    const float rho = bsA(F.B, g.nz, ck).z;
+    const bool thm = U.micro2.z > 0.5f;
+    const Fall fl{U.step.z, thm, U.hur3.w > 0.5f && !thm};
+    auto at = [&](float fall, int c) {
+      traceQH(U, F, g, par, kk, p, v, fall, 1.f, x, y, z);
+      sto(F.Qt[c], o, gatherQ(F.Q[0][c], tapQ(g, x, y, z)));
+    };
+    if (has(1)) sto(F.Qt[1], o, gatherQ(F.Q[0][1], t0));
+    if (has(7)) sto(F.Qt[7], o, gatherQ(F.Q[0][7], t0));
+    if (has(6) && !thm) sto(F.Qt[6], o, gatherQ(F.Q[0][6], t0));
+    if (has(2)) {
+      const float fi = vtI(U, ldo(F.Q[0][2], o), rho);
+      if (fi > 0.f) at(fi, 2);
+      else sto(F.Qt[2], o, gatherQ(F.Q[0][2], t0));
+    }
+    if (has(3) || (has(6) && thm)) {
+      const float2 fv = fl.vtRain(ldo(F.Q[0][3], o), ldo(F.Q[0][6], o), rho);
+      if (has(3)) at(fv.x, 3);
+      if (has(6) && thm) at(fv.y, 6);
+    }
+    if (has(4)) at(fl.vtS(ldo(F.Q[0][4], o), rho), 4);
+    if (has(5)) at(fl.vtGrau(ldo(F.Q[0][5], o), rho), 5);
+  }
+  const unsigned clear = kHydro & ~act & ~zeros;
+  if (clear) {
+#pragma unroll
+    for (int c = 1; c < 8; c++)
+      if ((clear >> c) & 1u) sto(F.Qt[c], o, 0.f);
+  }
 }
-__global__ void k_advq2_hur(Grid g, Uni U, Fields F) {
+__global__ void __launch_bounds__(128) k_advq2_hur(Grid g, Uni U, Fields F) {
   constexpr int par = 0;
-  brick_flags_all(g, F, nullptr, nullptr, F.zeroQ1);
   const int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y, ck = blockIdx.z;
+  const int brick = blockIdx.x + F.nbx * (blockIdx.y + F.nby * blockIdx.z);
+  const unsigned zeros = F.zeroQ1[brick];
+  const unsigned act = reach_channels(g, U, F, F.actQ0, F.actQt);
+  if (threadIdx.x == 0 && threadIdx.y == 0) F.zeroQ1[brick] = kHydro & ~act;
   if (ci >= g.nx || cj >= g.ny || ck >= g.nz) return;
-  const int o = g.at(ci, cj, ck);
+  auto has = [&](int c) { return ((act >> c) & 1u) != 0u; };
+  const unsigned o = 4u * unsigned(g.at(ci, cj, ck));
   const float kk[3] = {U.der.x, U.der.x, U.der.y};
   const float p[3] = {float(ci) + 0.5f, float(cj) + 0.5f, float(ck) + 0.5f};
   float v[3];
   cellVel(F, g, par, ci, cj, ck, v);
-  const float rho = bsA(F.B, g.nz, ck).z;
-  const bool thm = U.micro2.z > 0.5f;
-  const Fall fl{U.step.z, thm, U.hur3.w > 0.5f && !thm};
-  float q[8];
-#pragma unroll
-  for (int c = 0; c < 8; c++) q[c] = __ldg(F.Q[0][c] + o);
-  const float2 fv = fl.vtRain(q[3], q[6], rho);
-  const float fs = fl.vtS(q[4], rho), fg = fl.vtGrau(q[5], rho), fi = vtI(U, q[2], rho);
-  const float fn = thm ? fv.y : 0.f;
   const float cx = v[0] * kk[0], cy = v[1] * kk[1], cz = v[2] * kk[2];
   const float cour = sqrtf(cx * cx + cy * cy + cz * cz);
   const float sm = 0.5f * U.misc.y * clampf(cour / 0.35f, U.dzv.w, 1.f);
-  // each channel's fall speed (0: the air's)
-  const float fall[8] = {0.f, 0.f, fi, fv.x, fs, fg, fn, 0.f};
+  // channel c from its forward tap in the scratch, limited by the window of its departure tap
+  auto put = [&](int c, const Tap& tb, const Tap& tf) {
+    const float b = gatherQ(F.Qt[c], tb);
+    const float r = ldo(F.Qt[c], o) + sm * (ldo(F.Q[0][c], o) - b);
+    const float2 m = minmaxQ(F.Q[0][c], tf);
+    sto(F.Q[1][c], o, fmaxf(clampf(r, m.x, m.y), 0.f));
+  };
   float x, y, z;
+  auto tap = [&](float fall, float s) {
+    traceQH(U, F, g, par, kk, p, v, fall, s, x, y, z);
+    return tapQ(g, x, y, z);
+  };
+  const bool thm = U.micro2.z > 0.5f;
+  const float rho = bsA(F.B, g.nz, ck).z;
+  const float fi = has(2) ? vtI(U, ldo(F.Q[0][2], o), rho) : 0.f;
+  {  // at the air's speed
+    const Tap tb = tap(0.f, -1.f), tf = tap(0.f, 1.f);
+    put(0, tb, tf);
+    if (has(1)) put(1, tb, tf);
+    if (has(2) && fi == 0.f) put(2, tb, tf);
+    if (has(6) && !thm) put(6, tb, tf);
+    if (has(7)) put(7, tb, tf);
+  }
+  if (act & 0x7cu) {
+    const Fall fl{U.step.z, thm, U.hur3.w > 0.5f && !thm};
+    auto falling = [&](int c, float fall) {
+      const Tap tb = tap(fall, -1.f), tf = tap(fall, 1.f);
+      put(c, tb, tf);
+    };
+    if (has(2) && fi != 0.f) falling(2, fi);
+    if (has(3) || (has(6) && thm)) {
+      const float2 fv = fl.vtRain(ldo(F.Q[0][3], o), ldo(F.Q[0][6], o), rho);
+      if (has(3)) falling(3, fv.x);
+      if (has(6) && thm) falling(6, fv.y);
+    }
+    if (has(4)) falling(4, fl.vtS(ldo(F.Q[0][4], o), rho));
+    if (has(5)) falling(5, fl.vtGrau(ldo(F.Q[0][5], o), rho));
+  }
+  const unsigned clear = kHydro & ~act & ~zeros;
+  if (clear) {
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    traceQH(U, F, g, par, kk, p, v, fall[c], -1.f, x, y, z);
-    const float b = gatherQ(F.Qt[c], tapQ(g, x, y, z));
-    const float r = __ldg(F.Qt[c] + o) + sm * (q[c] - b);
-    traceQH(U, F, g, par, kk, p, v, fall[c], 1.f, x, y, z);
-    const float2 m = minmaxQ(F.Q[0][c], tapQ(g, x, y, z));
-    F.Q[1][c][o] = fmaxf(clampf(r, m.x, m.y), 0.f);
+    for (int c = 1; c < 8; c++)
+      if ((clear >> c) & 1u) sto(F.Q[1][c], o, 0.f);
   }
 }
 
@@ -1635,6 +1706,8 @@ void launch_advq(const Grid& g, const Uni& U, const Fields& F, int par, cudaStre
 }
 void launch_prep(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
   k_prep<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
+  cudaMemsetAsync(F.vmax, 0, 3 * sizeof(unsigned), s);
+  k_wind_max<<<592, 256, 0, s>>>(g, facing(F, par));
 }
 void launch_filt(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s) {
   k_filt<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
@@ -1648,7 +1721,8 @@ void launch_tables(const Grid& g, const Uni& U, const Fields& F, cudaStream_t s)
 }
 void launch_phys(const Grid& g, const Uni& U, const Fields& F, int par, cudaStream_t s, int micro_mode) {
   if (U.hur.x > 0.5f) {  // hurricane mode runs the scheme (model.js:578-907 with its hurricane branches)
-    k_phys_hur<<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
+    if (U.cor.z > 0.5f) k_phys_hur<1><<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
+    else k_phys_hur<0><<<grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3), kB3, 0, s>>>(g, U, facing(F, par));
     return;
   }
   const dim3 grid = grid3(g.nx + 1, g.ny + 1, g.nz + 1, kB3);
