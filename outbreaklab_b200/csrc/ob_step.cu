@@ -296,40 +296,47 @@ __global__ void k_init(Grid g, Uni U, Fields F) {
 template <bool HUR = false>
 __device__ __forceinline__ void nut_body(const Grid& g, const Uni& U, const Fields& F, int par, const int BX, const int BY, const int BZ) {
   OB_TEXEL_LOOP_BEGIN(g.nx - 1, g.ny - 1, g.nz - 1)
-  // a cell's +1 neighbours on the staggered box always exist; the -1 ones clamp to the edge (offset 0)
-  const int o = g.at(ci, cj, ck);
-  const int xm = ci > 0 ? -1 : 0, ym = cj > 0 ? -g.px : 0, zm = ck > 0 ? -g.plane : 0;
-  const int xp = 1, yp = g.px, zp = g.plane;
-  const float* __restrict__ u = F.V[par][0] + o;
-  const float* __restrict__ v = F.V[par][1] + o;
-  const float* __restrict__ w = F.V[par][2] + o;
-  const float* __restrict__ th = F.V[par][3] + o;
+  // a cell's +1 neighbours on the staggered box always exist; the -1 ones clamp to the edge
+  const unsigned o = 4u * unsigned(g.at(ci, cj, ck)), sy = 4u * unsigned(g.px), sz = 4u * unsigned(g.plane);
+  const unsigned xm = ci > 0 ? o - 4u : o, ym = cj > 0 ? o - sy : o, zm = ck > 0 ? o - sz : o;
+  const unsigned xp = o + 4u, yp = o + sy, zp = o + sz;
+  const float* __restrict__ u = F.V[par][0];
+  const float* __restrict__ v = F.V[par][1];
+  const float* __restrict__ w = F.V[par][2];
+  const float* __restrict__ th = F.V[par][3];
   const float u0m = bsB(F.B, g.nz, ck - 1).z, u00 = bsB(F.B, g.nz, ck).z, u0p = bsB(F.B, g.nz, ck + 1).z;
   const float v0m = bsB(F.B, g.nz, ck - 1).w, v00 = bsB(F.B, g.nz, ck).w, v0p = bsB(F.B, g.nz, ck + 1).w;
-  auto uc = [&](int off, float u0) { return 0.5f * (__ldg(u + off) + __ldg(u + off + xp)) - u0; };
-  auto vc = [&](int off, float v0) { return 0.5f * (__ldg(v + off) + __ldg(v + off + yp)) - v0; };
-  auto wc = [&](int off) { return 0.5f * (__ldg(w + off) + __ldg(w + off + zp)); };
+  auto uc = [&](unsigned at, float u0) { return 0.5f * (ldo(u, at) + ldo(u + 1, at)) - u0; };
+  auto vc = [&](unsigned at, float v0) { return 0.5f * (ldo(v, at) + ldo(v, at + sy)) - v0; };
+  auto wc = [&](unsigned at) { return 0.5f * (ldo(w, at) + ldo(w, at + sz)); };
   const float dx = U.dims.w, dz = U.dzv.x;
   // differences times the correctly rounded reciprocals 1/dx, 1/dz (and their exact halves) instead of divisions
   const float idx = U.dzv.y, idz = U.dzv.z, ih2x = 0.5f * idx, ih2z = 0.5f * idz;
-  const float dudx = (__ldg(u + xp) - __ldg(u)) * idx;
-  const float dvdy = (__ldg(v + yp) - __ldg(v)) * idx;
-  const float dwdz = (__ldg(w + zp) - __ldg(w)) * idz;
+  const float dudx = (ldo(u + 1, o) - ldo(u, o)) * idx;
+  const float dvdy = (ldo(v, yp) - ldo(v, o)) * idx;
+  const float dwdz = (ldo(w, zp) - ldo(w, o)) * idz;
   const float dudy = (uc(yp, u00) - uc(ym, u00)) * ih2x, dudz = (uc(zp, u0p) - uc(zm, u0m)) * ih2z;
   const float dvdx = (vc(xp, v00) - vc(xm, v00)) * ih2x, dvdz = (vc(zp, v0p) - vc(zm, v0m)) * ih2z;
   const float dwdx = (wc(xp) - wc(xm)) * ih2x, dwdy = (wc(yp) - wc(ym)) * ih2x;
   const float s12 = 0.5f * (dudy + dvdx), s13 = 0.5f * (dudz + dwdx), s23 = 0.5f * (dvdz + dwdy);
   const float S2 = 2.f * (dudx * dudx + dvdy * dvdy + dwdz * dwdz) + 4.f * (s12 * s12 + s13 * s13 + s23 * s23);
   const int kz0 = max(ck - 1, 0), kz1 = min(ck + 1, g.nz - 1);
-  float N2 = 9.81f / bsA(F.B, g.nz, ck).x * (__ldg(th + (kz1 - ck) * g.plane) - __ldg(th + (kz0 - ck) * g.plane)) / (float(kz1 - kz0) * dz);
-  if (U.cor.w > 0.5f && __ldg(F.Q[0][1] + o) + __ldg(F.Q[0][2] + o) > 1e-5f) N2 = fminf(N2, 0.f);
-  const float Ri = N2 / fmaxf(S2, 1e-10f);
-  const float fst = sqrtf(fmaxf(0.f, 1.f - Ri / 0.33f));
-  const float sS = sqrtf(fmaxf(S2, 0.f));
-  const float lh = U.turb.x * dx, lv = 0.18f * dz;
+  float N2 = 9.81f / bsA(F.B, g.nz, ck).x * (ldo(th, o + unsigned(kz1 - ck) * sz) - ldo(th, o + unsigned(kz0 - ck) * sz)) / (float(kz1 - kz0) * dz);
+  if (U.cor.w > 0.5f && ldo(F.Q[0][1], o) + ldo(F.Q[0][2], o) > 1e-5f) N2 = fminf(N2, 0.f);
   const float dtc = fmaxf(U.step.x, 0.1f);
-  F.aux[0][o] = fminf(lh * lh * sS * fst, 0.08f * dx * dx / dtc);
-  float nuv = fminf(lv * lv * sS * fst, 0.15f * dz * dz / dtc);
+  // Ri clearly past the critical value: the Richardson factor and both viscosities are exactly zero, as the divisions and
+  // roots below would find (a stable, weakly sheared cell; most are). An infinite S2 or a NaN takes the full form.
+  float nuh = 0.f, nuv = 0.f;
+  const float S2c = fmaxf(S2, 1e-10f);
+  if (!(N2 > 0.331f * S2c)) {
+    const float Ri = N2 / S2c;
+    const float fst = sqrtf(fmaxf(0.f, 1.f - Ri / 0.33f));
+    const float sS = sqrtf(fmaxf(S2, 0.f));
+    const float lh = U.turb.x * dx, lv = 0.18f * dz;
+    nuh = fminf(lh * lh * sS * fst, 0.08f * dx * dx / dtc);
+    nuv = fminf(lv * lv * sS * fst, 0.15f * dz * dz / dtc);
+  }
+  sto(F.aux[0], o, nuh);
   if (HUR) {  // hurricane mode: a K-profile boundary layer (model.js:377-386)
     const float zc = (float(ck) + 0.5f) * dz, h = U.hur2.z;
     if (zc < h) {
@@ -342,7 +349,7 @@ __device__ __forceinline__ void nut_body(const Grid& g, const Uni& U, const Fiel
       nuv = fmaxf(nuv, fminf(0.4f * ust * zc * q * q, 0.15f * dz * dz / dtc));
     }
   }
-  F.aux[1][o] = nuv;
+  sto(F.aux[1], o, nuv);
 }
 __global__ void __launch_bounds__(128, 16) k_nut(Grid g, Uni U, Fields F) { nut_body(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
 __global__ void k_nut_hur(Grid g, Uni U, Fields F) { nut_body<true>(g, U, F, 0, blockIdx.x, blockIdx.y, blockIdx.z); }
@@ -821,34 +828,35 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
   unsigned hyd = 0u;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int o = g.at(ci, cj, ck);
-  const float* __restrict__ Vu = F.V[1 - par][0] + o;
-  const float* __restrict__ Vv = F.V[1 - par][1] + o;
-  const float* __restrict__ Vw = F.V[1 - par][2] + o;
-  const float* __restrict__ Vth = F.V[1 - par][3] + o;
-  const float* __restrict__ A0 = F.aux[0] + o;
-  const float* __restrict__ A1 = F.aux[1] + o;
+  const unsigned b = unsigned(o) * 4u, sy = unsigned(g.px) * 4u, sz = unsigned(g.plane) * 4u;
+  const float* __restrict__ Vu = F.V[1 - par][0];
+  const float* __restrict__ Vv = F.V[1 - par][1];
+  const float* __restrict__ Vw = F.V[1 - par][2];
+  const float* __restrict__ Vth = F.V[1 - par][3];
+  const float* __restrict__ A0 = F.aux[0];
+  const float* __restrict__ A1 = F.aux[1];
   // staggered box
-  const int xm = ci > 0 ? -1 : 0, xp = ci < nx ? 1 : 0;
-  const int ym = cj > 0 ? -g.px : 0, yp = cj < ny ? g.px : 0;
-  const int zm = ck > 0 ? -g.plane : 0, zp = ck < nz ? g.plane : 0;
+  const unsigned xm = ci > 0 ? b - 4u : b, xp = ci < nx ? b + 4u : b;
+  const unsigned ym = cj > 0 ? b - sy : b, yp = cj < ny ? b + sy : b;
+  const unsigned zm = ck > 0 ? b - sz : b, zp = ck < nz ? b + sz : b;
   // cell box: own index and +-1, clamped to [0, n-1]
-  const int xc0 = ci < nx ? 0 : -1, xcp = ci < nx - 1 ? 1 : xc0;
-  const int yc0 = cj < ny ? 0 : -g.px, ycp = cj < ny - 1 ? g.px : yc0;
-  auto LP = [&](int off) {
+  const unsigned xc0 = ci < nx ? b : b - 4u, xcp = ci < nx - 1 ? b + 4u : xc0;
+  const unsigned yc0 = cj < ny ? b : b - sy, ycp = cj < ny - 1 ? b + sy : yc0;
+  auto LP = [&](unsigned at) {
     if (!BND) return 0.f;
-    return __ldg(F.phT + o + off);
+    return ldo(F.phT, at);
   };
   const float dx = U.dims.w, dz = U.dzv.x, dt = U.step.x;
-  float V[4] = {__ldg(Vu), __ldg(Vv), __ldg(Vw), __ldg(Vth)};
+  float V[4] = {ldo(Vu, b), ldo(Vv, b), ldo(Vw, b), ldo(Vth, b)};
   float out[4] = {V[0], V[1], V[2], V[3]};
   const float ix2 = U.der.z, iz2 = U.der.w;
   const float fc = U.cor.x;
   const float* __restrict__ Vc[4] = {Vu, Vv, Vw, Vth};
-  auto lapH = [&](int ch, float me) { return __ldg(Vc[ch] + xp) + __ldg(Vc[ch] + xm) + __ldg(Vc[ch] + yp) + __ldg(Vc[ch] + ym) - 4.f * me; };
+  auto lapH = [&](int ch, float me) { return ldo(Vc[ch], xp) + ldo(Vc[ch], xm) + ldo(Vc[ch], yp) + ldo(Vc[ch], ym) - 4.f * me; };
   auto lapZp = [&](int ch, float me, bool lo, bool hi) {
     const float m0 = me - bsV(F.B, nz, ck, ch);
-    const float a = lo ? m0 : __ldg(Vc[ch] + zm) - bsV(F.B, nz, ck - 1, ch);
-    const float b = hi ? m0 : __ldg(Vc[ch] + zp) - bsV(F.B, nz, ck + 1, ch);
+    const float a = lo ? m0 : ldo(Vc[ch], zm) - bsV(F.B, nz, ck - 1, ch);
+    const float b = hi ? m0 : ldo(Vc[ch], zp) - bsV(F.B, nz, ck + 1, ch);
     return a + b - 2.f * m0;
   };
   const float4 spk = __ldg(reinterpret_cast<const float4*>(F.spz) + ck);  // (top sponge centre, face, rain factor, -)
@@ -856,11 +864,11 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
   const float2 sly = __ldg(reinterpret_cast<const float2*>(F.sly) + cj);
   // u
   if (cj < ny && ck < nz) {
-    const float nux = 0.5f * (__ldg(A0 + xm) + __ldg(A0 + xc0)) + U.turb.y;
-    const float nuy = 0.5f * (__ldg(A1 + xm) + __ldg(A1 + xc0)) + U.turb.y;
+    const float nux = 0.5f * (ldo(A0, xm) + ldo(A0, xc0)) + U.turb.y;
+    const float nuy = 0.5f * (ldo(A1, xm) + ldo(A1, xc0)) + U.turb.y;
     float du = nux * lapH(0, V[0]) * ix2 + nuy * lapZp(0, V[0], ck == 0, ck == nz - 1) * iz2;
     const float ut = tgtUb<BND>(F, g, dz, ci, cj, ck);
-    const float vbar = 0.25f * (__ldg(Vv + xm) + V[1] + __ldg(Vv + xm + yp) + __ldg(Vv + yp));
+    const float vbar = 0.25f * (ldo(Vv, xm) + V[1] + ldo(Vv, xm + yp - b) + ldo(Vv, yp));
     const float vtb = 0.5f * (tgtVb<BND>(F, g, dz, ci - 1, cj, ck) + tgtVb<BND>(F, g, dz, ci, cj + 1, ck));
     const float sp = fmaxf(slx.x, sly.y) + spk.x;
     if (BND) {
@@ -870,7 +878,7 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
       du += sp * (ut - V[0]);
     }
     du += fc * (vbar - vtb);
-    if (BND && ci > 0 && ci < nx) du -= (LP(0) - LP(-1)) / dx;
+    if (BND && ci > 0 && ci < nx) du -= (LP(b) - LP(b - 4u)) / dx;
     if (ck == 0 && U.turb.w > 0.5f) {
       float cd = U.micro.w;
       if (HUR) {  // sea / land drag (model.js:649-652)
@@ -883,11 +891,11 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
   } else out[0] = 0.f;
   // v
   if (ci < nx && ck < nz) {
-    const float nux = 0.5f * (__ldg(A0 + ym) + __ldg(A0 + yc0)) + U.turb.y;
-    const float nuy = 0.5f * (__ldg(A1 + ym) + __ldg(A1 + yc0)) + U.turb.y;
+    const float nux = 0.5f * (ldo(A0, ym) + ldo(A0, yc0)) + U.turb.y;
+    const float nuy = 0.5f * (ldo(A1, ym) + ldo(A1, yc0)) + U.turb.y;
     float dv = nux * lapH(1, V[1]) * ix2 + nuy * lapZp(1, V[1], ck == 0, ck == nz - 1) * iz2;
     const float vt = tgtVb<BND>(F, g, dz, ci, cj, ck);
-    const float ubar = 0.25f * (__ldg(Vu + ym) + V[0] + __ldg(Vu + xp + ym) + __ldg(Vu + xp));
+    const float ubar = 0.25f * (ldo(Vu, ym) + V[0] + ldo(Vu, xp + ym - b) + ldo(Vu, xp));
     const float utb = 0.5f * (tgtUb<BND>(F, g, dz, ci, cj - 1, ck) + tgtUb<BND>(F, g, dz, ci + 1, cj, ck));
     const float sp = fmaxf(slx.y, sly.x) + spk.x;
     if (BND) {
@@ -897,7 +905,7 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
       dv += sp * (vt - V[1]);
     }
     dv -= fc * (ubar - utb);
-    if (BND && cj > 0 && cj < ny) dv -= (LP(0) - LP(-g.px)) / dx;
+    if (BND && cj > 0 && cj < ny) dv -= (LP(b) - LP(b - sy)) / dx;
     if (ck == 0 && U.turb.w > 0.5f) {
       float cd = U.micro.w;
       if (HUR) {
@@ -910,21 +918,21 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
   } else out[1] = 0.f;
   // w
   if (ci < nx && cj < ny && ck > 0 && ck < nz) {
-    const float nux = 0.5f * (__ldg(A0 - g.plane) + __ldg(A0)) + U.turb.y;
-    const float nuy = 0.5f * (__ldg(A1 - g.plane) + __ldg(A1)) + U.turb.y;
-    float dw = nux * lapH(2, V[2]) * ix2 + nuy * (__ldg(Vw - g.plane) + __ldg(Vw + g.plane) - 2.f * V[2]) * iz2;
-    auto buoy = [&](int kk, int off) {
+    const float nux = 0.5f * (ldo(A0, b - sz) + ldo(A0, b)) + U.turb.y;
+    const float nuy = 0.5f * (ldo(A1, b - sz) + ldo(A1, b)) + U.turb.y;
+    float dw = nux * lapH(2, V[2]) * ix2 + nuy * (ldo(Vw, b - sz) + ldo(Vw, b + sz) - 2.f * V[2]) * iz2;
+    auto buoy = [&](int kk, unsigned at) {
       const float4 A = bsA(F.B, nz, kk);
       float h[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
       if (!dry) {
 #pragma unroll
-        for (int c = 0; c < 5; c++) h[c] = __ldg(F.Q[1][1 + c] + o + off);
+        for (int c = 0; c < 5; c++) h[c] = ldo(F.Q[1][1 + c], at);
       }
-      return 9.81f * ((__ldg(Vth + off) - A.x) / A.x + 0.608f * (__ldg(F.Q[1][0] + o + off) - A.y) -
+      return 9.81f * ((ldo(Vth, at) - A.x) / A.x + 0.608f * (ldo(F.Q[1][0], at) - A.y) -
                       (h[0] + h[1] + h[2] + h[3] + h[4]));
     };
-    dw += 0.5f * (buoy(ck - 1, -g.plane) + buoy(ck, 0));
-    if (BND) dw -= (LP(0) - LP(-g.plane)) / dz;
+    dw += 0.5f * (buoy(ck - 1, b - sz) + buoy(ck, b));
+    if (BND) dw -= (LP(b) - LP(b - sz)) / dz;
     dw += (fmaxf(slx.y, sly.y) + spk.y) * (0.f - V[2]);
     const float4 civ = __ldg(F.ciMap + cj * nx + ci);
     if (!HUR && civ.x > 0.f) {  // hurricane mode starts storms as warm bubbles instead (model.js:686-687)
@@ -944,25 +952,25 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
     const float tth = BND ? tgtTh(F.B, g, dz, LAv, ck) : A.x, tqv = BND ? tgtQv(F.B, g, dz, LAv, ck) : A.y;
     const float sl = fmaxf(slx.y, sly.y);
     const float relax = BND ? sl + l2d(F.lsfB, g, ci, cj).w * (1.f / U.cor.y) : sl;
-    const float nux = __ldg(A0) * 3.f + U.turb.y, nuy = __ldg(A1) * 3.f + U.turb.y;
+    const float nux = ldo(A0, b) * 3.f + U.turb.y, nuy = ldo(A1, b) * 3.f + U.turb.y;
     float th = V[3] + dt * (nux * lapH(3, V[3]) * ix2 + nuy * lapZp(3, V[3], ck == 0, ck == nz - 1) * iz2 + (relax + spk.x) * (tth - V[3]));
     // hydrometeor and spare channels: exactly +0 throughout a dry block's reach, so not read there (the sums below
     // then see the same +0 operands the loads would have returned)
-    float q1[4] = {__ldg(F.Q[1][0] + o), 0.f, 0.f, 0.f}, q2[4] = {0.f, 0.f, 0.f, 0.f};
+    float q1[4] = {ldo(F.Q[1][0], b), 0.f, 0.f, 0.f}, q2[4] = {0.f, 0.f, 0.f, 0.f};
     float l1[3] = {0.f, 0.f, 0.f}, l1z[3] = {0.f, 0.f, 0.f};
     if (!dry) {
 #pragma unroll
       for (int c = 0; c < 4; c++) {
-        if (c) q1[c] = __ldg(F.Q[1][c] + o);
-        q2[c] = __ldg(F.Q[1][4 + c] + o);
+        if (c) q1[c] = ldo(F.Q[1][c], b);
+        q2[c] = ldo(F.Q[1][4 + c], b);
       }
     }
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       if (c && dry) continue;
-      const float* __restrict__ q = F.Q[1][c] + o;
-      l1[c] = __ldg(q + xcp) + __ldg(q + xm) + __ldg(q + ycp) + __ldg(q + ym) - 4.f * q1[c];
-      l1z[c] = (ck == 0 ? q1[c] : __ldg(q + zm)) + (ck == nz - 1 ? q1[c] : __ldg(q + g.plane)) - 2.f * q1[c];
+      const float* __restrict__ q = F.Q[1][c];
+      l1[c] = ldo(q, xcp) + ldo(q, xm) + ldo(q, ycp) + ldo(q, ym) - 4.f * q1[c];
+      l1z[c] = (ck == 0 ? q1[c] : ldo(q, zm)) + (ck == nz - 1 ? q1[c] : ldo(q, b + sz)) - 2.f * q1[c];
     }
     const float qvb = (ck == 0 ? A.y : bsA(F.B, nz, ck - 1).y) + (ck == nz - 1 ? A.y : bsA(F.B, nz, ck + 1).y) - 2.f * A.y;
     l1z[0] -= qvb;
@@ -1004,7 +1012,7 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
       if (ck == 0) {  // the sea's sensible and latent heat; dissipative heating
         const float4 sf = __ldg(F.sfc + cj * nx + ci);
         const float land = clampf(sf.x, 0.f, 1.f);
-        const float ua = 0.5f * (V[0] + __ldg(Vu + 1)), va = 0.5f * (V[1] + __ldg(Vv + g.px));
+        const float ua = 0.5f * (V[0] + ldo(Vu, b + 4u)), va = 0.5f * (V[1] + ldo(Vv, b + sy));
         const float u1 = sqrtf(ua * ua + va * va);
         const float ch = U.hur.y * U.hur2.w * fmaxf(u1, U.hur3.y) / dz;
         const float ps = fmaxf(U.hur.w + A.z * U.cn.y * __ldg(F.phi + g.pidx(ci, cj, ck)), 50000.f);
@@ -1076,29 +1084,32 @@ __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, cons
       const float keep = HUR ? 1.f / (1.f + 2.f * dt * sl + dt * envDecay) : (sl > 0.f ? 1.f / (1.f + 2.f * dt * sl) : 1.f);
       qc *= keep; qi *= keep; qr *= keep; qs *= keep; qg *= keep; nr *= keep;
       const float nv[8] = {0.f, qc, qi, qr, qs, qg, thm ? nr : q2[2], q2[3]};
-      F.Q[0][0][o] = fmaxf(qv, 0.f);
+      sto(F.Q[0][0], b, fmaxf(qv, 0.f));
       const bool any = qc > 0.f || qi > 0.f || qr > 0.f || qs > 0.f || qg > 0.f || nv[6] > 0.f || nv[7] > 0.f;
       if (any || old) {  // else the channels below are zero here and slot 0 already holds zeros
 #pragma unroll
         for (int c = 1; c < 8; c++) {
           if (nv[c] > 0.f) hyd |= 1u << c;
-          if (nv[c] > 0.f || ((old >> c) & 1u)) F.Q[0][c][o] = c == 7 ? nv[c] : fmaxf(nv[c], 0.f);
+          if (nv[c] > 0.f || ((old >> c) & 1u)) sto(F.Q[0][c], b, c == 7 ? nv[c] : fmaxf(nv[c], 0.f));
         }
       }
       out[3] = th;
     }
   }
-  const float sp = sqrtf(out[0] * out[0] + out[1] * out[1] + out[2] * out[2]);
-  if (sp > U.misc.x) {
-    const float s = U.misc.x / sp;
-    out[0] *= s; out[1] *= s; out[2] *= s;
+  const float s2 = out[0] * out[0] + out[1] * out[1] + out[2] * out[2];
+  if (s2 > 0.999f * U.misc.x * U.misc.x) {   // no root for a speed below the cap
+    const float sp = sqrtf(s2);
+    if (sp > U.misc.x) {
+      const float s = U.misc.x / sp;
+      out[0] *= s; out[1] *= s; out[2] *= s;
+    }
   }
   if (!(out[0] == out[0]) || !(out[1] == out[1]) || !(out[2] == out[2]) || !(out[3] == out[3])) {
     out[0] = bsB(F.B, nz, ck).z; out[1] = bsB(F.B, nz, ck).w; out[2] = 0.f; out[3] = bsA(F.B, nz, ck).x;
     atomicAdd(F.flags, 1u);
   }
 #pragma unroll
-  for (int c = 0; c < 4; c++) F.V[par][c][o] = out[c];
+  for (int c = 0; c < 4; c++) sto(F.V[par][c], b, out[c]);
   return hyd;
 }
 
