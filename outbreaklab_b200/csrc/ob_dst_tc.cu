@@ -71,6 +71,78 @@ __device__ __forceinline__ void prefetch_rows(const TcOut& out, int m, int n0, i
   for (int c = n0; c < c1; c += 32) tc::prefetch_l2(row + c);
   tc::prefetch_l2(row + c1);
 }
+
+// One chunk of the product, field row m (this lane's) x outputs c0 .. c0 + 31 in v, to global memory; outputs from cend on
+// and rows from M on (!mv) are not written. Transposed modes write a column at a time, 32 consecutive field rows by the
+// warp's lanes; row modes turn the chunk in shared memory (stg, 32 x STG_LD floats of this warp), so that a store (and a
+// load of the old values) covers 32 consecutive outputs of a row. base: the lane's element of output 0 (transposed modes);
+// mrow: the warp's first row. The four epilogue warps are alone on their schedulers and bounded the transforms: 19 instructions
+// a value went to a test and a 64-bit address each, and the last tile's rows were loaded, added and stored one after the
+// other. A whole chunk is stored without tests, addresses step by the pitch and all loads come first. Pair kernel, plain
+// bf16 / bf16x3: 198 -> 170 us / 348 -> 316 us at 1024 x 1024 x 80 (what is left is the operands' way out of L2, 7.6 TB/s,
+// and the tensor cores); 49 -> 37 us / 68 -> 61 us at 640 x 640 x 40; the added rows of a 203 x 157 x 40 step 20 -> 18 us.
+template <int MODE, bool ONE>
+__device__ __forceinline__ void store_chunk(const TcOut& out, const float (&v)[32], long base, int c0, int cend, bool mv, int mrow, int lane,
+                                            float* stg) {
+  long ld = out.ld;
+  asm volatile("" : "+l"(ld));   // its multiples are stepped through, not kept in 64 registers across the chunks
+  if (MODE == OUT_T_BF16X2 || MODE == OUT_T_F32) {
+    if (!mv) return;
+    const long a = base + long(c0) * ld;
+    float* f = MODE == OUT_T_F32 ? out.f + a : nullptr;
+    __nv_bfloat16* hi = MODE == OUT_T_F32 ? nullptr : out.hi + a;
+    __nv_bfloat16* lo = MODE == OUT_T_F32 || ONE ? nullptr : out.lo + a;   // the next transform of a plain-bf16 pass reads hi alone
+    auto put = [&](float x) {
+      if (MODE == OUT_T_F32) {
+        *f = x;
+        f += ld;
+      } else if (ONE) {
+        *hi = __float2bfloat16_rn(x);
+        hi += ld;
+      } else {
+        tc::split_bf16(x, *hi, *lo);
+        hi += ld;
+        lo += ld;
+      }
+    };
+    if (c0 + 32 <= cend) {
+#pragma unroll
+      for (int c = 0; c < 32; c++) put(v[c]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 32; c++)
+        if (c0 + c < cend) put(v[c]);
+    }
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < 32; c++) stg[lane * STG_LD + c] = v[c];
+  __syncwarp();
+  const bool cv = c0 + lane < cend;
+  if (cv) {
+    float* const p = out.f + long(mrow) * ld + c0 + lane;
+    const int rows = out.M - mrow;   // below 32 in the last tile alone
+    float old[32], val[32];
+    auto drain = [&](auto there) {
+      if (MODE == OUT_R_F32_ADD) {
+        const float* o = p;
+#pragma unroll
+        for (int r = 0; r < 32; r++, o += ld) old[r] = there(r) ? *o : 0.f;
+      }
+      // every staged value read before the first store, so that the 32 row stores issue back to back
+#pragma unroll
+      for (int r = 0; r < 32; r++) val[r] = stg[r * STG_LD + lane];
+      float* w = p;
+#pragma unroll
+      for (int r = 0; r < 32; r++, w += ld)
+        if (there(r)) *w = MODE == OUT_R_F32_ADD ? old[r] + val[r] : val[r];
+    };
+    if (rows >= 32) drain([](int) { return true; });
+    else drain([&](int r) { return r < rows; });
+  }
+  __syncwarp();
+}
+
 }  // namespace
 
 // one tile of a transform: its operands, sizes and output, and its corner
@@ -269,55 +341,14 @@ __device__ __forceinline__ void dst_tc_run(const Src& src, unsigned int* err) {
       const bool mv = m < out.M;
       const int cend = min(out.N, n0 + BN);  // columns past BN belong to the next tile (BN need not be a multiple of 32)
       const int plane = m / out.R, r = m - plane * out.R;
+      const long base = long(plane) * out.N * out.ld + r;
       for (int ch = 0; ch * 32 < BN; ch++) {
         float v[32];
         tc::tmem_ld32(tmem + uint32_t(b * 256) + (uint32_t(q * 32) << 16) + uint32_t(ch * 32), v);
         const int c0 = n0 + ch * 32;
         if (c0 >= cend) continue;
-        if (MODE == OUT_T_BF16X2 || MODE == OUT_T_F32) {
-          // column by column: the warp's 32 lanes write 32 consecutive field rows of one output row
-          if (mv) {
-            const long base = long(plane) * out.N * out.ld + r;
-#pragma unroll
-            for (int c = 0; c < 32; c++) {
-              if (c0 + c < cend) {
-                const long a = base + long(c0 + c) * out.ld;
-                if (MODE == OUT_T_F32) {
-                  out.f[a] = v[c];
-                } else if (ONE) {  // the next transform of a plain-bf16 pass reads the hi plane alone
-                  out.hi[a] = __float2bfloat16_rn(v[c]);
-                } else {
-                  __nv_bfloat16 h, l;
-                  tc::split_bf16(v[c], h, l);
-                  out.hi[a] = h;
-                  out.lo[a] = l;
-                }
-              }
-            }
-          }
-        } else {
-          // row-major output: the warp's 32 rows x 32 columns go through shared memory so that each store (and,
-          // when adding, each load of the old values) covers one row's 32 consecutive columns: 128 bytes
-          float* stg = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES + 256) + q * 32 * STG_LD;
-#pragma unroll
-          for (int c = 0; c < 32; c++) stg[lane * STG_LD + c] = v[c];
-          __syncwarp();
-          const bool cv = c0 + lane < cend;
-          const int mrow = m0 + q * 32;
-          float old[32];
-          if (MODE == OUT_R_F32_ADD) {
-#pragma unroll
-            for (int r = 0; r < 32; r++) old[r] = (cv && mrow + r < out.M) ? out.f[long(mrow + r) * out.ld + c0 + lane] : 0.f;
-          }
-#pragma unroll
-          for (int r = 0; r < 32; r++) {
-            if (cv && mrow + r < out.M) {
-              const float val = stg[r * STG_LD + lane];
-              out.f[long(mrow + r) * out.ld + c0 + lane] = MODE == OUT_R_F32_ADD ? old[r] + val : val;
-            }
-          }
-          __syncwarp();
-        }
+        store_chunk<MODE, ONE>(out, v, base, c0, cend, mv, m0 + q * 32, lane,
+                               reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES + 256) + q * 32 * STG_LD);
       }
       // the accumulator is free again once every lane's tcgen05.ld of it has completed
       tc::tc_fence_before();
@@ -549,52 +580,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int m = m0 + q * 32 + lane;
       const bool mv = m < out.M;
       const int plane = m / out.R, r = m - plane * out.R;
+      const long base = long(plane) * out.N * out.ld + r;
       for (int ch = 0; ch * 32 < BN; ch++) {   // a sub-tile's chunks past its end are skipped below
         float v[32];
         tc::tmem_ld32(tmem + uint32_t(b * 256) + (uint32_t(q * 32) << 16) + uint32_t(ch * 32), v);
         const int c0 = n0 + ch * 32;
         if (c0 >= cend) continue;
-        if (MODE == OUT_T_BF16X2 || MODE == OUT_T_F32) {
-          if (mv) {
-            const long base = long(plane) * out.N * out.ld + r;
-#pragma unroll
-            for (int c = 0; c < 32; c++) {
-              if (c0 + c < cend) {
-                const long a = base + long(c0 + c) * out.ld;
-                if (MODE == OUT_T_F32) {
-                  out.f[a] = v[c];
-                } else if (ONE) {
-                  out.hi[a] = __float2bfloat16_rn(v[c]);
-                } else {
-                  __nv_bfloat16 h, l;
-                  tc::split_bf16(v[c], h, l);
-                  out.hi[a] = h;
-                  out.lo[a] = l;
-                }
-              }
-            }
-          }
-        } else {
-          float* stg = reinterpret_cast<float*>(smem) + q * 32 * STG_LD;
-#pragma unroll
-          for (int c = 0; c < 32; c++) stg[lane * STG_LD + c] = v[c];
-          __syncwarp();
-          const bool cv = c0 + lane < cend;
-          const int mrow = m0 + q * 32;
-          float old[32];
-          if (MODE == OUT_R_F32_ADD) {
-#pragma unroll
-            for (int rr = 0; rr < 32; rr++) old[rr] = (cv && mrow + rr < out.M) ? out.f[long(mrow + rr) * out.ld + c0 + lane] : 0.f;
-          }
-          // every staged value read before the first store, so that the 32 row stores issue back to back
-          float val[32];
-#pragma unroll
-          for (int rr = 0; rr < 32; rr++) val[rr] = stg[rr * STG_LD + lane];
-#pragma unroll
-          for (int rr = 0; rr < 32; rr++)
-            if (cv && mrow + rr < out.M) out.f[long(mrow + rr) * out.ld + c0 + lane] = MODE == OUT_R_F32_ADD ? old[rr] + val[rr] : val[rr];
-          __syncwarp();
-        }
+        store_chunk<MODE, ONE>(out, v, base, c0, cend, mv, m0 + q * 32, lane, reinterpret_cast<float*>(smem) + q * 32 * STG_LD);
       }
       // the accumulator is free again once both CTAs' epilogue warps have read it
       tc::tc_fence_before();
