@@ -756,7 +756,8 @@ __device__ __forceinline__ float tri_pivot_rcp(const float4& o, float shift, flo
 //   1. one 3-D TMA load brings the block's [NZ][16][16] fp32 tile of T2[k][m][l] into shared memory (zero outside);
 //   2. each thread runs the Thomas sweep of its mode: c' in registers, d and then x updated in place in the tile
 //      (a warp's tile row is 32 consecutive floats: no bank conflicts), the 2 x 2 lowest modes in FP64 with the
-//      host-factored coefficients. The z-operator (lower, upper, diagonal, rhoC per level) is a kernel parameter,
+//      host-factored coefficients, which their block fetches while its tile is in flight: that one block is the last to
+//      end, and a load from L2 every few levels of its chain made it 14 us of a small launch (10 us now, 80 x 80 x 40). The z-operator (lower, upper, diagonal, rhoC per level) is a kernel parameter,
 //      so every coefficient is a constant-bank operand of the instruction that uses it (no load in the recurrence),
 //      and the reciprocal of each pivot is the hardware's rcp.approx (at most 1 ulp from the rounded quotient);
 //   3. one barrier later every thread reads the NZ/8 half rows (level, l, 8 m) it will write, splits them into bf16
@@ -771,7 +772,7 @@ __device__ __forceinline__ float tri_pivot_rcp(const float4& o, float shift, flo
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int TRI_TL = 16, TRI_TM = 16;
 template <int NZ>
-constexpr int tri_smem_bytes() { return NZ * TRI_TM * TRI_TL * 4 + 4 * NZ * 8 /*FP64 low modes*/ + 128 /*align*/ + 16 /*barrier*/; }
+constexpr int tri_smem_bytes() { return NZ * TRI_TM * TRI_TL * 4 + 12 * NZ * 8 /*FP64 low modes and their factors*/ + 128 /*align*/ + 16 /*barrier*/; }
 // the z-operator by value: (lower, upper, diagonal, rhoC) of each level (solver.js:139-146)
 template <int NZ>
 struct TriZ {
@@ -787,7 +788,8 @@ __device__ __forceinline__ void tri_tma_tile(const CUtensorMap* tIn, const CUten
   static_assert(NZ % 8 == 0, "levels come in whole groups of 8");
   float* tile = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(smraw) + 127) & ~uintptr_t(127));
   double* dlow = reinterpret_cast<double*>(tile + NZ * TRI_TM * TRI_TL);   // [4][NZ]: d of the FP64 low modes
-  uint64_t* bar = reinterpret_cast<uint64_t*>(dlow + 4 * NZ);
+  double* coef = dlow + 4 * NZ;                                            // [4][2][NZ]: their factors (low)
+  uint64_t* bar = reinterpret_cast<uint64_t*>(coef + 8 * NZ);
   static_assert(TRI_TL == 16 && TRI_TM == 16, "thread and output mappings below assume 16 x 16 modes");
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, tid = threadIdx.x;
   if (tid == 0) {
@@ -806,6 +808,8 @@ __device__ __forceinline__ void tri_tma_tile(const CUtensorMap* tIn, const CUten
   const bool act = l < nxp && m < nyp;
   // what the sweep needs besides the tile, fetched while the tile is in flight
   const float shift = act ? __ldg(lam + l) + __ldg(lam + nxp + m) : 0.f;
+  if (l0 == 0 && m0 == 0)
+    for (int t = tid; t < 8 * NZ; t += TRI_TL * TRI_TM) coef[t] = __ldg(low + t);
   // one thread waits (bounded) for the tile and tells the others; if it never arrived the error word reports it and
   // every thread leaves before touching the tile
   __shared__ int s_ok;
@@ -839,20 +843,20 @@ __device__ __forceinline__ void tri_tma_tile(const CUtensorMap* tIn, const CUten
   } else if (act) {
     // lowest modes: low[(mode*2 + 0)*NZ + k] = 1/den_k, low[(mode*2 + 1)*NZ + k] = c'_k (FP64, host-factored)
     const int mode = m * 2 + l;
-    const double* rd = low + (mode * 2) * NZ;
+    const double* rd = coef + (mode * 2) * NZ;
     const double* cpd = rd + NZ;
     double* d = dlow + mode * NZ;
     double dprev = 0.0;
 #pragma unroll 8
-    for (int k = 0; k < NZ; k++) {   // the coefficient loads do not depend on the recurrence: unrolled, they overlap
-      dprev = (double(col[k * LS]) - double(zop(k).x) * dprev) * __ldg(rd + k);
+    for (int k = 0; k < NZ; k++) {
+      dprev = (double(col[k * LS]) - double(zop(k).x) * dprev) * rd[k];
       d[k] = dprev;
     }
     double x = dprev;
     col[(NZ - 1) * LS] = float(x);
 #pragma unroll 8
     for (int k = NZ - 2; k >= 0; k--) {
-      x = d[k] - __ldg(cpd + k) * x;
+      x = d[k] - cpd[k] * x;
       col[k * LS] = float(x);
     }
   } else {
