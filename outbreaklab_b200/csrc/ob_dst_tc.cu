@@ -79,8 +79,8 @@ __device__ __forceinline__ void prefetch_rows(const TcOut& out, int m, int n0, i
 // mrow: the warp's first row. The four epilogue warps are alone on their schedulers and bounded the transforms: 19 instructions
 // a value went to a test and a 64-bit address each, and the last tile's rows were loaded, added and stored one after the
 // other. A whole chunk is stored without tests, addresses step by the pitch and all loads come first. Pair kernel, plain
-// bf16 / bf16x3: 198 -> 170 us / 348 -> 316 us at 1024 x 1024 x 80 (what is left is the operands' way out of L2, 7.6 TB/s,
-// and the tensor cores); 49 -> 37 us / 68 -> 61 us at 640 x 640 x 40; the added rows of a 203 x 157 x 40 step 20 -> 18 us.
+// bf16 / bf16x3: 198 -> 170 us / 348 -> 316 us at 1024 x 1024 x 80 (tensor pipe 43 -> 50 % and 84 -> 90 % busy);
+// 49 -> 37 us / 68 -> 61 us at 640 x 640 x 40; the added rows of a 203 x 157 x 40 step 20 -> 18 us.
 template <int MODE, bool ONE>
 __device__ __forceinline__ void store_chunk(const TcOut& out, const float (&v)[32], long base, int c0, int cend, bool mv, int mrow, int lane,
                                             float* stg) {
