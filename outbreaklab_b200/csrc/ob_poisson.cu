@@ -305,8 +305,6 @@ static int ck(cudaError_t e, const char* what) {
   return OB_OK;
 }
 
-static void fp32_attrs();
-
 int PoissonPlan::create(int nx_, int ny_, int nz_, double dx_, double dz_, int precision_) {
   nx = nx_; ny = ny_; nz = nz_; dx = dx_; dz = dz_; precision = precision_;
   if (nx < 2 || ny < 2 || nz < 2 || nz > 4096) { set_error("poisson: bad size %d x %d x %d", nx, ny, nz); return OB_ERR_INVALID; }
@@ -336,7 +334,7 @@ int PoissonPlan::create(int nx_, int ny_, int nz_, double dx_, double dz_, int p
   if ((rc = ck(cudaMalloc(&lam, lamh.size() * sizeof(float)), "poisson eig"))) return rc;
   if ((rc = ck(cudaMalloc(&zop, size_t(nz) * sizeof(float4)), "poisson zop"))) return rc;
   if (precision == 0) {   // the tensor-core precisions hold their fields in the buffers of tc_create
-    fp32_attrs();
+    if ((rc = fp32_prepare())) return rc;
     if ((rc = ck(cudaMalloc(&tmp, n * sizeof(float)), "poisson tmp"))) return rc;
     if ((rc = ck(cudaMalloc(&hat, n * sizeof(float)), "poisson hat"))) return rc;
     if ((rc = ck(cudaMalloc(&cpd, size_t(8) * nz * sizeof(double)), "poisson low-mode scratch"))) return rc;
@@ -382,13 +380,15 @@ static void launch_gemm(int M, int N, int K, const float* mat, const float* src,
   const int rt = (M + 32 * GR - 1) / (32 * GR), ct = (N + 16 * CPT - 1) / (16 * CPT);
   k_gemm_f32<XT, GR, CPT><<<unsigned(rt) * unsigned(ct), GTH, gemm_smem_bytes<GR, CPT>(), s>>>(M, N, K, mat, src, dst, nx, pl, XT ? rt : ct);
 }
-// on every create: a function's attributes belong to the device that is current
-static void fp32_attrs() {
-  cudaFuncSetAttribute(k_gemm_f32<true, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 8>());
-  cudaFuncSetAttribute(k_gemm_f32<true, 3, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<3, 8>());
-  cudaFuncSetAttribute(k_gemm_f32<false, 4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 8>());
-  cudaFuncSetAttribute(k_gemm_f32<false, 4, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<4, 6>());
-  cudaFuncSetAttribute(k_tri_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, kTriSmemLevels * kTriThreads * 8);
+// a function's attributes belong to the device that is current
+int fp32_prepare() {
+  const auto smem = [](auto* k, int bytes) { return ck(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "poisson fp32 kernels"); };
+  int rc = smem(k_gemm_f32<true, 4, 8>, gemm_smem_bytes<4, 8>());
+  if (rc == OB_OK) rc = smem(k_gemm_f32<true, 3, 8>, gemm_smem_bytes<3, 8>());
+  if (rc == OB_OK) rc = smem(k_gemm_f32<false, 4, 8>, gemm_smem_bytes<4, 8>());
+  if (rc == OB_OK) rc = smem(k_gemm_f32<false, 4, 6>, gemm_smem_bytes<4, 6>());
+  if (rc == OB_OK) rc = smem(k_tri_f32, kTriSmemLevels * kTriThreads * 8);
+  return rc;
 }
 // x-transform (solver.js mode 0): dst(l, col) = sum_i M(l, i) src(i, col), col = j + ny k
 void PoissonPlan::gemm_x(const float* Mx, const float* src, float* dst, cudaStream_t s) const {

@@ -47,6 +47,10 @@ struct PoissonPlan {
   void tc_destroy();
 };
 
+// lets the fp32 solve's kernels (gemm_x, gemm_y, tri) have their shared memory on the current device: called before the
+// first of them there, by create and by whoever uses a plan without it
+int fp32_prepare();
+
 // FP64 residual norms of phi for rhs (device arrays) under the solve's operator: rel = {max |r| / max |rhs|,
 // ||r||_2 / ||rhs||_2}; scratch holds 4 * 1024 + 4 doubles
 int poisson_residual(const PoissonPlan& P, const float* rhs, const float* phi, double* scratch, double rel[2], cudaStream_t s);

@@ -93,7 +93,8 @@ extern "C" int ob_poisson_solve_static(int nx, int ny, int nz, float dx, float d
   }
   float* base = nullptr;
   {
-    // first call on this device: look up the array's device address (must happen before any stream capture)
+    // first call on this device: look up the array's device address (must happen before any stream capture) and give the
+    // kernels their shared memory, since no plan may ever be created here
     std::lock_guard<std::mutex> lk(g_static_mu);
     if (!g_static_ptr[dev]) {
       e = cudaGetSymbolAddress(reinterpret_cast<void**>(&base), g_poisson_scratch);
@@ -101,6 +102,8 @@ extern "C" int ob_poisson_solve_static(int nx, int ny, int nz, float dx, float d
         set_error("ob_poisson_solve_static: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
         return OB_ERR_DEVICE;
       }
+      const int rc = fp32_prepare();
+      if (rc != OB_OK) return rc;
       g_static_ptr[dev] = base;
     }
     base = g_static_ptr[dev];
