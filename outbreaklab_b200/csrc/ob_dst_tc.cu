@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // any multiple of 4 bytes, the planes' rows at 16). Bound by memory: 1024 x 1024 x 80 in precision 5, which needs no lo plane, takes
 // 74 us (6.8 TB/s); a value per thread at a time, its row found by a 64-bit division and both planes written, took 225 us.
 template <bool LO, bool VEC>
-__global__ void __launch_bounds__(256) k_split_rows(const float* __restrict__ src, long rows, int cols, __nv_bfloat16* __restrict__ hi,
+__global__ void __launch_bounds__(256) k_split_rows(const float* src, long rows, int cols, __nv_bfloat16* __restrict__ hi,
                                                     __nv_bfloat16* __restrict__ lo, int ld) {
   tc::grid_wait();
   tc::grid_release();
@@ -621,11 +621,11 @@ __global__ void __launch_bounds__(256) k_split_rows(const float* __restrict__ sr
     for (int c = lane * 4; c < ld; c += 128) {   // ld is a multiple of 8
       float v[4];
       if (VEC && c + 4 <= cols) {
-        const float4 q = __ldg(reinterpret_cast<const float4*>(p + c));
+        const float4 q = tc::ld_late(reinterpret_cast<const float4*>(p + c));
         v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; e++) v[e] = c + e < cols ? __ldg(p + c + e) : 0.f;
+        for (int e = 0; e < 4; e++) v[e] = c + e < cols ? tc::ld_late(p + c + e) : 0.f;
       }
       __align__(8) __nv_bfloat16 h[4], l[4];
 #pragma unroll
@@ -641,25 +641,26 @@ __global__ void __launch_bounds__(256) k_split_rows(const float* __restrict__ sr
 // with phi = 0 on the faces beyond the grid (antisymmetric ghosts, the operator the sine transforms diagonalise) and
 // Neumann in z (lo = 0 at the ground, up = 0 at the lid); written split for the correction solve
 // ---------------------------------------------------------------------------------------------------------------
+// (phi is the transform's before it, under whose tail k_resid may start: ordinary loads)
 __device__ __forceinline__ void resid_body(int nx, int ny, int nz, double idx2, const float4* __restrict__ zop, const float* __restrict__ rhs,
-                                           const float* __restrict__ phi, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
+                                           const float* phi, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                            int ld, const int BX, const int BY, const int BZ) {
   const int i = BX * blockDim.x + threadIdx.x, j = BY, k = BZ;
   if (i >= nx) return;
   const long pl = long(nx) * ny;
   const long o = long(k) * pl + long(j) * nx + i;
-  const double p = phi[o];
-  const double xm = i > 0 ? double(phi[o - 1]) : -p, xp = i < nx - 1 ? double(phi[o + 1]) : -p;
-  const double ym = j > 0 ? double(phi[o - nx]) : -p, yp = j < ny - 1 ? double(phi[o + nx]) : -p;
+  const double p = tc::ld_late(phi + o);
+  const double xm = i > 0 ? double(tc::ld_late(phi + o - 1)) : -p, xp = i < nx - 1 ? double(tc::ld_late(phi + o + 1)) : -p;
+  const double ym = j > 0 ? double(tc::ld_late(phi + o - nx)) : -p, yp = j < ny - 1 ? double(tc::ld_late(phi + o + nx)) : -p;
   const float4 z = __ldg(zop + k);
-  const double zm = k > 0 ? double(phi[o - pl]) : 0.0, zp = k < nz - 1 ? double(phi[o + pl]) : 0.0;
+  const double zm = k > 0 ? double(tc::ld_late(phi + o - pl)) : 0.0, zp = k < nz - 1 ? double(tc::ld_late(phi + o + pl)) : 0.0;
   const double Lp = double(z.w) * (xm + xp + ym + yp - 4.0 * p) * idx2 + double(z.x) * zm + double(z.z) * p + double(z.y) * zp;
   const float r = float(double(rhs[o]) - Lp);
   const long t = (long(k) * ny + j) * ld + i;
   tc::split_bf16(r, hi[t], lo[t]);
 }
 __global__ void k_resid(int nx, int ny, int nz, double idx2, const float4* __restrict__ zop, const float* __restrict__ rhs,
-                        const float* __restrict__ phi, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int ld) {
+                        const float* phi, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int ld) {
   tc::grid_wait();   // no grid_release: from 1e5 blocks of four warps it doubles the kernel's time; the next kernel starts as they end
   resid_body(nx, ny, nz, idx2, zop, rhs, phi, hi, lo, ld, blockIdx.x, blockIdx.y, blockIdx.z);
 }

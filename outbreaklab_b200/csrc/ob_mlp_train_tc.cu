@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_mlp_step(const __grid_const
       tc::tmem_ld32(trow + uint32_t(ph * NH + c0), v);
 #pragma unroll
       for (int e = 0; e < 32; e++) {
-        const float z = v[e] + __ldg(bias + e);
+        const float z = v[e] + tc::ld_late(bias + e);
         v[e] = gelu(z);
         gp[e] = gelu_grad(z);
       }
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_mlp_step(const __grid_const
 #pragma unroll
           for (int e = 0; e < 16; e++) {
             float d = 0.f;
-            if (e < NLOSS) d = y[e] + __ldg(P.w + OB4 + e) - T[e < NLOSS ? e : 0];
+            if (e < NLOSS) d = y[e] + tc::ld_late(P.w + OB4 + e) - T[e < NLOSS ? e : 0];
             l += double(d) * d;
             dy[e] = P.inv * d;
           }
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(256) k_grad_adam(Parts S, float* __restrict__ 
   else { part = S.p[3]; N = NHX; j = t - OB4; n = NH; }
   float gi = 0.f;
 #pragma unroll 16
-  for (int z = 0; z < S.nsplit; z++) gi += part[(long(z) * GBM + j) * N + n];
+  for (int z = 0; z < S.nsplit; z++) gi += tc::ld_late(part + (long(z) * GBM + j) * N + n);
   g[t] = gi;
   if (!A.w) return;
   const float mi = A.b1 * A.m[t] + (1.f - A.b1) * gi, vi = A.b2 * A.v[t] + (1.f - A.b2) * gi * gi;

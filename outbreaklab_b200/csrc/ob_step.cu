@@ -14,6 +14,14 @@
 
 namespace ob {
 
+// reads of what the pass just before has written (ldo, gather8)
+using tc::ld_late;
+__device__ __forceinline__ float ldo_late(const float* f, unsigned b) { return ld_late(reinterpret_cast<const float*>(reinterpret_cast<const char*>(f) + b)); }
+__device__ __forceinline__ float gather8_late(const float* f, const Corners& t) {
+  return lerp8(t, ldo_late(f, t.a), ldo_late(f, t.b), ldo_late(f, t.c), ldo_late(f, t.d), ldo_late(f, t.e), ldo_late(f, t.h), ldo_late(f, t.k),
+               ldo_late(f, t.l));
+}
+
 // members of the grouped launches (ensemble steps), uploaded by group_upload_members. A grouped launch's grid is
 // (x-y blocks of all members, 1, levels): the members share nz, and blockIdx.x indexes a map that gives each x-y
 // block its member and its block coordinates (one 8-byte load per thread, the same for the whole block).
@@ -407,6 +415,12 @@ __device__ __forceinline__ float sampleVch(const float* f, const Grid& g, int ch
   return trilerpB(f, g, g.nx + 1, g.ny + 1, g.nz + 1, x - ox, y - oy, z - oz);
 }
 
+// the same from the scratch that ADVV1 has just written
+__device__ __forceinline__ float sampleVt(const Fields& F, const Grid& g, int ch, float x, float y, float z) {
+  const float ox = ch == 0 ? 0.f : 0.5f, oy = ch == 1 ? 0.f : 0.5f, oz = ch == 2 ? 0.f : 0.5f;
+  return gather8_late(F.Vt[ch], corners(g, g.nx + 1, g.ny + 1, g.nz + 1, x - ox, y - oy, z - oz));
+}
+
 // the departure-point sample of a channel, with the min / max of its 8 texels (ADVV2's limiter window: the
 // reference's limiter traces the same point, model.js:455-479)
 __device__ __forceinline__ void sampleVch_mm(const Fields& F, const Grid& g, int par, int ch, unsigned o, float x, float y, float z) {
@@ -454,10 +468,10 @@ __device__ __forceinline__ void advv2_body(const Grid& g, const Uni& U, const Fi
   for (int c = 0; c < 4; c++) {
     float x, y, z;
     traceV(g, kk, P[c][0], P[c][1], P[c][2], vel[c], -1.f, x, y, z);
-    const float b = sampleVch(F.Vt[c], g, c, x, y, z);
-    const float hat = ldo(F.Vt[c], o), old = ldo(F.V[par][c], o);
+    const float b = sampleVt(F, g, c, x, y, z);
+    const float hat = ldo_late(F.Vt[c], o), old = ldo(F.V[par][c], o);
     const float r = hat + sm * (old - b);
-    sto(F.V[1 - par][c], o, clampf(r, ldo(F.Vlo[c], o), ldo(F.Vhi[c], o)));
+    sto(F.V[1 - par][c], o, clampf(r, ldo_late(F.Vlo[c], o), ldo_late(F.Vhi[c], o)));
   }
 }
 __global__ void __launch_bounds__(128, 12) k_advv2(Grid g, Uni U, Fields F) {
@@ -551,7 +565,7 @@ __device__ __forceinline__ unsigned box_channels(const Grid& g, const Fields& F,
     const int bx = bx0 + t % nxb, by = by0 + (t / nxb) % nyb, bz = bz0 + t / (nxb * nyb);
     const int b = bx + F.nbx * (by + F.nby * bz);
     any |= __ldg(flagsA + b);
-    if (flagsB) any |= __ldg(flagsB + b);
+    if (flagsB) any |= ld_late(flagsB + b);   // those of ADVQ1, just before
   }
   any = __reduce_or_sync(0xffffffffu, any);
   if ((threadIdx.x & 31) == 0 && any) atomicOr(&held, any);
@@ -661,8 +675,8 @@ __device__ __forceinline__ float advq2_channel(const Fields& F, const Grid& g, c
                                                float fall, float sm, float qc_, int c, unsigned o) {
   float x, y, z;
   traceQ(g, kk, p, v, fall, -1.f, x, y, z);
-  const float b = gatherQ(F.Qt[c], tapQ(g, x, y, z));
-  const float r = ldo(F.Qt[c], o) + sm * (qc_ - b);
+  const float b = gather8_late(F.Qt[c], tapQ(g, x, y, z));
+  const float r = ldo_late(F.Qt[c], o) + sm * (qc_ - b);
   traceQ(g, kk, p, v, fall, 1.f, x, y, z);
   const float2 m = minmaxQ(F.Q[0][c], tapQ(g, x, y, z));
   return fmaxf(clampf(r, m.x, m.y), 0.f);
@@ -701,8 +715,8 @@ __device__ __forceinline__ void advq2_body(const Grid& g, const Uni& U, const Fi
     {  // the air-speed group: qv always; qc, qi, the spare channel and, in the Lin scheme, Nr where held
       const Tap tb = tapQ(g, xb, yb, zb), tf = tapQ(g, xf, yf, zf);
       auto air = [&](int c) {
-        const float b = gatherQ(F.Qt[c], tb);
-        const float rr = ldo(F.Qt[c], o) + sm * (ldo(F.Q[0][c], o) - b);
+        const float b = gather8_late(F.Qt[c], tb);
+        const float rr = ldo_late(F.Qt[c], o) + sm * (ldo(F.Q[0][c], o) - b);
         const float2 m = minmaxQ(F.Q[0][c], tf);
         sto(F.Q[1][c], o, fmaxf(clampf(rr, m.x, m.y), 0.f));
       };
@@ -1182,15 +1196,15 @@ __global__ void __launch_bounds__(128, 9) k_phys_grp(const uint2* __restrict__ m
 __device__ __forceinline__ void div_body(const Grid& g, const Uni& U, const Fields& F, int par, const int BX, const int BY, const int BZ) {
   OB_TEXEL_LOOP_BEGIN(g.nx - 1, g.ny - 1, g.nz - 1)
   const int o = g.at(ci, cj, ck);
-  const float* __restrict__ u = F.V[par][0];
-  const float* __restrict__ v = F.V[par][1];
-  const float* __restrict__ w = F.V[par][2];
+  const float* u = F.V[par][0];   // PHYS has just written these
+  const float* v = F.V[par][1];
+  const float* w = F.V[par][2];
   const float rc = bsA(F.B, g.nz, ck).z;
-  const float wt = ck == g.nz - 1 ? 0.f : __ldg(w + o + g.plane);
-  const float wb = ck == 0 ? 0.f : __ldg(w + o);
+  const float wt = ck == g.nz - 1 ? 0.f : ld_late(w + o + g.plane);
+  const float wb = ck == 0 ? 0.f : ld_late(w + o);
   // the reference divides by dx, dz and dt (model.js:909-925); multiplying by the host's reciprocals (1/dx, 1/dz in
   // dzv, 1/dt in der2) saves three IEEE divisions per cell and moves r by a few ulp
-  const float d = rc * (__ldg(u + o + 1) - __ldg(u + o) + __ldg(v + o + g.px) - __ldg(v + o)) * U.dzv.y +
+  const float d = rc * (ld_late(u + o + 1) - ld_late(u + o) + ld_late(v + o + g.px) - ld_late(v + o)) * U.dzv.y +
                   (rhoW(F.B, g.nz, ck + 1) * wt - rhoW(F.B, g.nz, ck) * wb) * U.dzv.z;
   const float r = d * U.der2.x;
   if (F.rhs_hi) {  // tensor-core solve: write the split directly in its [z][y][x] layout with pitch rhs_ld
@@ -1215,8 +1229,8 @@ __global__ void k_div_grp(const uint2* __restrict__ map, int par) {
 // ---------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void proj_body(const Grid& g, const Uni& U, const Fields& F, int par, const int BX, const int BY, const int BZ) {
   OB_TEXEL_LOOP_BEGIN(g.nx, g.ny, g.nz)
-  auto P = [&](int a, int b, int c) {
-    return __ldg(F.phi + g.pidx(clampi(a, -g.pad, g.nx + g.pad - 1), clampi(b, -g.pad, g.ny + g.pad - 1), clampi(c, 0, g.nz - 1)));
+  auto P = [&](int a, int b, int c) {   // the solve's last kernel has just written phi
+    return ld_late(F.phi + g.pidx(clampi(a, -g.pad, g.nx + g.pad - 1), clampi(b, -g.pad, g.ny + g.pad - 1), clampi(c, 0, g.nz - 1)));
   };
   const int o = g.at(ci, cj, ck);
   const float kx = U.der.x, kz = U.der.y;

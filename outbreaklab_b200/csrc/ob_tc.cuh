@@ -49,6 +49,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
 // kernel start setting itself up when all blocks have called it or left.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A value that the kernel before writes, in such a kernel: an ordinary load, kept behind grid_wait. The read-only path
+// (__ldg, or const __restrict__ where the compiler takes it for the same) is for data that no one writes while the kernel
+// runs, and this one runs from before the other's end.
+__device__ __forceinline__ float ld_late(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_late(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned ld_late(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 
 // a launch whose kernel, if early, sets itself up (barriers, TMEM, tensor maps) under the tail of the kernel before it in
 // the stream (grid_wait)
