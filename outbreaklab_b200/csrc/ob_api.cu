@@ -356,14 +356,21 @@ int ob_model_create(const ObGrid* grid, ObModel** out) {
     set_error("ob_model_create: bad grid %d x %d x %d, dx %g", nx, ny, nz, double(grid->dx));
     return OB_ERR_INVALID;
   }
+  // the kernels reach a field's values at unsigned 32-bit byte offsets (ldo); whether 47 of them and the solve's arrays fit
+  // the GPU is the allocations' to say
+  const double px = std::floor((nx + 32.0) / 32.0) * 32.0, py = ny + 1.0;
+  if (px * py * (nz + 1) * sizeof(float) > 4294967296.0) {
+    set_error("ob_model_create: grid too large (a field of %d x %d x %d takes more than 4 GiB)", nx, ny, nz);
+    return OB_ERR_INVALID;
+  }
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { set_error("ob_model_create: no CUDA device"); return OB_ERR_DEVICE; }
   ObModel* m = new ObModel();
   host_copy_retain();
   Grid& g = m->g;
   g.nx = nx; g.ny = ny; g.nz = nz;
-  g.px = ((nx + 1) + 31) / 32 * 32;
-  g.py = ny + 1;
+  g.px = int(px);
+  g.py = int(py);
   g.plane = g.px * g.py;
   g.pad = ob_grid_pad(grid->dx);
   g.nxp = nx + 2 * g.pad;
@@ -374,8 +381,6 @@ int ob_model_create(const ObGrid* grid, ObModel** out) {
   m->Ly = ny * m->dx;
   ob_params_default(&m->P);
   m->P.spongeW = float(std::fmin(std::fmax(0.08 * std::fmin(m->Lx, m->Ly), 5000.0), 40000.0));  // model.js:1207
-  const double fieldsz = double(g.plane) * (nz + 1);
-  if (fieldsz * 39 * 4 > 170e9) { delete m; host_copy_release(); set_error("ob_model_create: grid too large for one GPU"); return OB_ERR_INVALID; }
   const size_t fs = (size_t(g.plane) * (nz + 1) + 63) / 64 * 64;
   m->fs = fs;
   const size_t n2 = size_t(nx) * ny, np = size_t(g.nxp) * g.nyp * nz;

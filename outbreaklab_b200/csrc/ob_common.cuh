@@ -252,8 +252,8 @@ struct Fall {
 // shares it: the gathers' offsets then take one register each, where element indices were widened to a 64-bit address per
 // access (ADVV1 fits 32 registers and 16 blocks per SM; unsigned element offsets take fewer instructions still, but their
 // multiply-adds to 64 bits run at half rate: 102 us against 94 us for ADVV1). At 320 x 320 x 40: ADVV1 107 -> 94 us, ADVV2
-// 122 -> 114 us, ADVQ1 91 -> 80 us, ADVQ2 169 -> 146 us. A field array is under 4 GiB: 47 of them and the solve's fill the
-// GPU's memory at 3.8e9 bytes each.
+// 122 -> 114 us, ADVQ1 91 -> 80 us, ADVQ2 169 -> 146 us. A field array is 4 GiB at most: ob_model_create
+// refuses larger grids.
 __device__ __forceinline__ float ldo(const float* __restrict__ f, unsigned b) {
   return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(f) + b));
 }
