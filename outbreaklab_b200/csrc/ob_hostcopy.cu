@@ -8,8 +8,8 @@
 // threads 2.5-2.9 ms, with chunks of half the size or 12 threads no less.
 //
 // The ring is one per process (16 MiB), made at the first large copy and given back when the last model goes
-// (host_copy_release). A copy that finds it taken by another thread, made for another device, or not to be had goes the
-// driver's way.
+// (host_copy_release). A copy that finds it taken by another thread, made for another device, or not to be had, and one from
+// another device than the current one, goes the driver's way.
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -74,9 +74,11 @@ cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t 
   Ring& R = ring();
   int dev = -1;
   std::unique_lock<std::mutex> use(R.use, std::defer_lock);
-  cudaPointerAttributes at{};
+  cudaPointerAttributes at{}, from{};
   const bool ordinary = bytes >= kMinBytes && cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
-  if (!ordinary || cudaGetDevice(&dev) != cudaSuccess || !use.try_lock() || !R.make() || R.device != dev) {
+  // the ring's events belong to the device that is current when it is made, and are recorded on s
+  const bool here = ordinary && cudaGetDevice(&dev) == cudaSuccess && cudaPointerGetAttributes(&from, src) == cudaSuccess && from.device == dev;
+  if (!here || !use.try_lock() || !R.make() || R.device != dev) {
     const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
     return e != cudaSuccess ? e : cudaStreamSynchronize(s);
   }

@@ -6,8 +6,7 @@
 
 namespace ob {
 
-// copies bytes of device memory, as the work queued on s leaves it, into dst and waits for it (the caller's thread holds
-// the copy's device as its current one)
+// copies bytes of device memory, as the work queued on s leaves it, into dst and waits for it
 cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
 // the owners of the copies' pinned ring: it is freed with the last of them
 void host_copy_retain();
