@@ -13,9 +13,7 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 #include <thread>
-#include <vector>
 
 #include "ob_hostcopy.cuh"
 
@@ -115,7 +113,7 @@ cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t 
   int started = 1;
   try {
     for (; started < nt; started++) th[started] = std::thread(work, started);
-  } catch (const std::system_error&) {   // no more threads to be had: this one takes over their chunks below
+  } catch (...) {   // no more threads to be had, or no memory for them: this one takes over their chunks below
   }
   for (int t = started; t < nt; t++) work(t);
   work(0);

@@ -46,6 +46,7 @@ inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void
 """
 
 HEAD = r"""
+#include <algorithm>
 #include <cstdio>
 #include <new>
 #include <vector>
@@ -100,3 +101,34 @@ int main() {
 }
 """)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_no_memory_for_the_threads(tmp_path):
+    """Any failure to start the draining threads leaves their chunks to the caller's thread; nothing escapes a C entry."""
+    r = _run(tmp_path, r"""
+static thread_local int fail_in = -1;   // allocations of this thread until one fails (-1: none does)
+void* operator new(size_t n) {
+  if (fail_in == 0) throw std::bad_alloc();
+  if (fail_in > 0) fail_in--;
+  if (void* p = std::malloc(n)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+int main() {
+  const size_t n = (size_t(21) << 20) + 12;
+  fill(n);
+  std::vector<uint8_t> out(n);
+  ob::host_copy_retain();
+  for (int k = 0; k < 9; k++) {
+    std::fill(out.begin(), out.end(), uint8_t(7));
+    fail_in = k;
+    const cudaError_t e = ob::copy_to_host(out.data(), fake_mem[0], n, &stream[0]);
+    fail_in = -1;
+    if (e != cudaSuccess || out != mem[0]) { std::printf("allocation %d\n", k); return 1; }
+  }
+  ob::host_copy_release();
+  return 0;
+}
+""")
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
