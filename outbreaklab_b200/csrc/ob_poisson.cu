@@ -50,24 +50,24 @@ constexpr int gemm_smem_bytes() { return GST * GBK * (32 * GR + 4 + 16 * CPT + 4
 // otherwise y-transform. Rows = (k, i) of the field: R(r, q) = src[i + nx q + pl k]; columns = outputs m of the matrix
 //     My[m][q], C[i + nx m + pl k].
 template <bool XT, int GR, int CPT>
-__global__ void __launch_bounds__(GTH, 2) k_gemm_f32(int M, int N, int K, const float* __restrict__ mat, const float* __restrict__ src,
-                                                     float* __restrict__ C, int nx, long pl, int mtiles) {
-  static_assert(XT || GR == 4, "the y-transform loads one field row per thread");
-  constexpr int BR = 32 * GR, BC = 16 * CPT, LR = BR + 4, LC = BC + 4, STG = GBK * (LR + LC);
+__global__ void __launch_bounds__(GTH, GR == 2 ? 4 : 2)
+    k_gemm_f32(int M, int N, int K, const float* __restrict__ mat, const float* __restrict__ src, float* __restrict__ C, int nx, long pl, int mtiles) {
+  static_assert(XT || GTH % (32 * GR) == 0, "the y-transform loads one field row per thread");
+  constexpr int BR = 32 * GR, BC = 16 * CPT, LR = BR + 4, LC = BC + 4, STG = GBK * (LR + LC), YQ = GTH / BR;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lx = lane & 7, ly = lane >> 3;
   // the matrix's tiles vary fastest, so that blocks running together share a field tile through L2
   const int bm = int(blockIdx.x % unsigned(mtiles)), bf = int(blockIdx.x / unsigned(mtiles));
   const int r0 = (XT ? bm : bf) * BR, c0 = (XT ? bf : bm) * BC;
   // this thread's cp.async lines: K-contiguous operands take (q = tid & 15, 8 lines per pass); the y-transform's field
-  // rows take row tid, one q-value per pass
+  // rows take row tid % BR, YQ q-values per pass
   const int kq = tid & 15, kl = tid >> 4;
   const float* rbase;   // rows operand
   bool rin = true;
   if (XT) {
     rbase = mat + long(r0 + kl) * K + kq;
   } else {
-    const int r = r0 + tid;
+    const int r = r0 + tid % BR;
     rin = r < M;
     const int k = r / nx, i = r - k * nx;
     rbase = src + (rin ? long(k) * pl + i : 0);
@@ -85,9 +85,10 @@ __global__ void __launch_bounds__(GTH, 2) k_gemm_f32(int M, int N, int K, const 
       }
     } else {
 #pragma unroll
-      for (int p = 0; p < GBK; p++) {
-        const bool in = rin && q0 + p < K;
-        cp_async4(s + p * LR + tid, in ? rbase + long(q0 + p) * nx : src, in);
+      for (int p = 0; p < GBK; p += YQ) {
+        const int q = YQ == 1 ? p : p + tid / BR;
+        const bool in = rin && q0 + q < K;
+        cp_async4(s + q * LR + tid % BR, in ? rbase + long(q0 + q) * nx : src, in);
       }
     }
     float* sc = s + GBK * LR;
@@ -375,6 +376,16 @@ void PoissonPlan::destroy() {
 
 // the width of the tiles that span n outputs of a DST matrix: 96 where that pads n less than 128 does
 static bool narrow_tiles(int n) { return (n + 95) / 96 * 96 < (n + 127) / 128 * 128; }
+// Tiles of 64 x 64 with 8 x 4 outputs per thread, where the wide ones would leave a third of the 148 SMs without a block: a
+// block's time is then all there is, and a quarter of the outputs take a quarter of it. Whole solves, wide -> small: 128 x
+// 128 x 28 (28 wide tiles) 103 -> 53 us, 64 x 64 x 56 (28) 74 -> 53, 64 x 300 x 28 (66 and 42) 122 -> 64, 192 x 192 x 28 (84)
+// 108 -> 84, 224 x 224 x 28 (98) 144 -> 125; from there on the wide tiles' fewer reads of shared memory tell: 256 x 256 x
+// 28 (112) 159 -> 167, 464 x 464 x 60 (1090) 1165 -> 1428.
+constexpr int kFewTiles = 98;
+static bool small_tiles(int n, int rows) {
+  const int t = narrow_tiles(n) ? 96 : 128;
+  return long((n + t - 1) / t) * ((rows + 127) / 128) <= kFewTiles;
+}
 template <bool XT, int GR, int CPT>
 static void launch_gemm(int M, int N, int K, const float* mat, const float* src, float* dst, int nx, long pl, cudaStream_t s) {
   const int rt = (M + 32 * GR - 1) / (32 * GR), ct = (N + 16 * CPT - 1) / (16 * CPT);
@@ -392,13 +403,15 @@ int fp32_prepare() {
 }
 // x-transform (solver.js mode 0): dst(l, col) = sum_i M(l, i) src(i, col), col = j + ny k
 void PoissonPlan::gemm_x(const float* Mx, const float* src, float* dst, cudaStream_t s) const {
-  if (narrow_tiles(nx)) launch_gemm<true, 3, 8>(nx, ny * nz, nx, Mx, src, dst, nx, 0, s);
+  if (small_tiles(nx, ny * nz)) launch_gemm<true, 2, 4>(nx, ny * nz, nx, Mx, src, dst, nx, 0, s);
+  else if (narrow_tiles(nx)) launch_gemm<true, 3, 8>(nx, ny * nz, nx, Mx, src, dst, nx, 0, s);
   else launch_gemm<true, 4, 8>(nx, ny * nz, nx, Mx, src, dst, nx, 0, s);
 }
 // y-transform (mode 1), per plane k: dst(i, m) = sum_j src(i, j) M(m, j)
 void PoissonPlan::gemm_y(const float* My, const float* src, float* dst, cudaStream_t s) const {
   const long pl = long(nx) * ny;
-  if (narrow_tiles(ny)) launch_gemm<false, 4, 6>(nx * nz, ny, ny, My, src, dst, nx, pl, s);
+  if (small_tiles(ny, nx * nz)) launch_gemm<false, 2, 4>(nx * nz, ny, ny, My, src, dst, nx, pl, s);
+  else if (narrow_tiles(ny)) launch_gemm<false, 4, 6>(nx * nz, ny, ny, My, src, dst, nx, pl, s);
   else launch_gemm<false, 4, 8>(nx * nz, ny, ny, My, src, dst, nx, pl, s);
 }
 void PoissonPlan::tri(float* h, cudaStream_t s) const {
