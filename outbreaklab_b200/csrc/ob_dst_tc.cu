@@ -79,8 +79,8 @@ __device__ __forceinline__ void prefetch_rows(const TcOut& out, int m, int n0, i
 // mrow: the warp's first row. The four epilogue warps are alone on their schedulers and bounded the transforms: 19 instructions
 // a value went to a test and a 64-bit address each, and the last tile's rows were loaded, added and stored one after the
 // other. A whole chunk is stored without tests, addresses step by the pitch and all loads come first. Pair kernel, plain
-// bf16 / bf16x3: 198 -> 170 us / 348 -> 316 us at 1024 x 1024 x 80 (tensor pipe 43 -> 50 % and 84 -> 90 % busy);
-// 49 -> 37 us / 68 -> 61 us at 640 x 640 x 40; the added rows of a 203 x 157 x 40 step 20 -> 18 us.
+// bf16 / bf16x3: 198 -> 171 us / 343 -> 326 us at 1024 x 1024 x 80 (tensor pipe 43 -> 50 % and 84 -> 90 % busy);
+// 49 -> 37 us / 67 -> 62 us at 656 x 656 x 40; the added rows of a 203 x 157 x 40 step 20 -> 18 us.
 template <int MODE, bool ONE>
 __device__ __forceinline__ void store_chunk(const TcOut& out, const float (&v)[32], long base, int c0, int cend, bool mv, int mrow, int lane,
                                             float* stg) {
@@ -119,23 +119,30 @@ __device__ __forceinline__ void store_chunk(const TcOut& out, const float (&v)[3
   for (int c = 0; c < 32; c++) stg[lane * STG_LD + c] = v[c];
   __syncwarp();
   const bool cv = c0 + lane < cend;
-  if (cv) {
+  float val[32];
+  if (MODE == OUT_R_F32) {
+    // every staged value read before the first store, so that the 32 row stores issue back to back. An address and a test
+    // each here: stepping as below took 194 us against 188 us (1024 x 1024 x 80, plain bf16) and 42.1 against 41.4 us (656 x
+    // 656 x 40), without a difference below that
+#pragma unroll
+    for (int r = 0; r < 32; r++) val[r] = stg[r * STG_LD + lane];
+#pragma unroll
+    for (int r = 0; r < 32; r++)
+      if (cv && mrow + r < out.M) out.f[long(mrow + r) * out.ld + c0 + lane] = val[r];
+  } else if (cv) {
     float* const p = out.f + long(mrow) * ld + c0 + lane;
     const int rows = out.M - mrow;   // below 32 in the last tile alone
-    float old[32], val[32];
+    float old[32];
     auto drain = [&](auto there) {
-      if (MODE == OUT_R_F32_ADD) {
-        const float* o = p;
+      const float* o = p;
 #pragma unroll
-        for (int r = 0; r < 32; r++, o += ld) old[r] = there(r) ? *o : 0.f;
-      }
-      // every staged value read before the first store, so that the 32 row stores issue back to back
+      for (int r = 0; r < 32; r++, o += ld) old[r] = there(r) ? *o : 0.f;
 #pragma unroll
       for (int r = 0; r < 32; r++) val[r] = stg[r * STG_LD + lane];
       float* w = p;
 #pragma unroll
       for (int r = 0; r < 32; r++, w += ld)
-        if (there(r)) *w = MODE == OUT_R_F32_ADD ? old[r] + val[r] : val[r];
+        if (there(r)) *w = old[r] + val[r];
     };
     if (rows >= 32) drain([](int) { return true; });
     else drain([&](int r) { return r < rows; });
