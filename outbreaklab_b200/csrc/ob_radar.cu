@@ -227,10 +227,13 @@ __device__ GateOut gate(const RadarU& R, const Grid& g, const Fields& F, int par
 
 // What the scan of a cut needs of its trigonometry, worked out on the host in 64 bits: the sines of the elevation at the
 // beam's three points, its cosine, and the site's up, north and east vectors in the frame (east, north, up) of the
-// projection's centre.
+// projection's centre. all: no gate may be left out, because the cut comes within 6 degrees of a pole, where gatePos takes its
+// position from an arc sine near 1 and an arc tangent of two small numbers: their rounding moves it by about a metre over the
+// cosine of the latitude, which is past the scan's margin within 2 degrees.
 struct ScanU {
   float se, sl, su, ce;
   float3 up, north, east;
+  bool all;
 };
 static ScanU scan_uniforms(const RadarU& R) {
   const double p0 = R.geo.x, p1 = R.geo.z, dl = double(R.geo.w) - double(R.geo.y), el = R.cut.x, q = 0.4 * 0.0165;
@@ -245,6 +248,7 @@ static ScanU scan_uniforms(const RadarU& R) {
   S.north = f3(-std::sin(p1) * std::sin(dl), std::cos(p0) * std::cos(p1) + std::sin(p0) * std::sin(p1) * std::cos(dl),
                std::sin(p0) * std::cos(p1) - std::cos(p0) * std::sin(p1) * std::cos(dl));
   S.east = f3(std::cos(dl), std::sin(p0) * std::sin(dl), -std::cos(p0) * std::sin(dl));
+  S.all = !(std::fabs(p1) + (double(R.gates.z) + double(R.gates.w) * double(R.gates.x)) / 6371000.0 <= 1.466);
   return S;
 }
 // Whether a gate can come out anything but empty: false only if gate() leaves it empty, whatever its last bits. The
@@ -255,6 +259,7 @@ static ScanU scan_uniforms(const RadarU& R) {
 // and every write of the scalars remake them), then the rain, snow and graupel themselves. Out of these alone each
 // reflectivity is +0, and with no tornado about there is no debris, so the echo is below any floor.
 __device__ __forceinline__ bool may_echo(const RadarU& R, const ScanU& S, const Grid& g, const Fields& F, int ri, int gi) {
+  if (S.all) return true;
   const float r = R.gates.z + R.gates.w * float(gi);
   const float az = (R.cut.y + R.cut.z * float(ri)) * 0.017453293f;
   const float dx = R.mdl.w, dz = R.mdl2.x, zAnt = R.site.z - R.mdl2.y, a = R.site.w;
