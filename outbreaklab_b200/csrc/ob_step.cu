@@ -1276,20 +1276,30 @@ __global__ void k_rain_grp(const uint2* __restrict__ map, int par) {
 // ---------------------------------------------------------------------------------------------------------------
 // WGSL_M_MAP (model.js:1028-1100): 16 diagnostics per column
 // ---------------------------------------------------------------------------------------------------------------
-// A block takes 32 columns of a row (one brick wide); its eight warps share the levels, kMapLevels at a time. What needs
-// an order (the updraft-helicity sum upwards, the cloud-top radiance downwards) leaves its terms in shared memory for
-// the first warp to add in that order; the maxima need none. Levels whose brick holds no precipitation have -30 dBZ and
-// levels without any hydrometeor are transparent (F.actQ0). One thread per column spent its time
-// on the latency of nz levels in turn: 72 -> 22 us at 64 x 64 x 40, 74 -> 33 us at 203 x 157 x 40; from 320 x 320 on, where
-// there are threads enough either way, 112 -> 96 us at 56 levels and no change at 640 x 640 (0.25 ms).
-constexpr int kMapWarps = 8, kMapLevels = 32;
+// A warp takes 32 columns of a row (one brick wide) and W of them share the levels, 4 W at a time; a block of eight has 8 / W
+// rows. What needs an order (the updraft-helicity sum upwards, the cloud-top radiance downwards) leaves its terms in
+// shared memory for the first of the W to add in that order, so W changes no bit; the maxima need none. Levels whose brick
+// holds no precipitation have -30 dBZ and levels without any hydrometeor are transparent (F.actQ0). One thread per column
+// (column "1 thread", 2-D blocks) spends its time on the latency of nz levels in turn; but the sums and what follows them
+// are left to one warp in W, which tells where there are warps enough without sharing. us:
+//                    1 thread   W = 8      4      2      1
+//   64 x 64 x 40         36.6    13.6   19.0   29.2   51.5
+//   203 x 157 x 16       16.8    14.2   11.7   15.1   22.8
+//   260 x 260 x 40       60.6    36.5   36.7   38.2   56.1
+//   400 x 380 x 40       97.6    94.1   77.6   76.2   87.7
+//   640 x 640 x 40      241     252    213    190    213
+//   900 x 900 x 16      174     291    208    173    159
+// (lin scheme, a storm every 60 km)
+constexpr int kMapWarps = 8;
+template <int W>
 __global__ void __launch_bounds__(32 * kMapWarps) k_maps(Grid g, Uni U, Fields F, float4* out) {
-  constexpr int par = 0;
-  __shared__ float s_uh[kMapLevels][32], s_a[kMapLevels][32], s_t[kMapLevels][32];
+  constexpr int par = 0, R = kMapWarps / W, LV = 4 * W;
+  __shared__ float s_uh[R][LV][32], s_a[R][LV][32], s_t[R][LV][32];
   __shared__ float s_max[2][kMapWarps][32];
-  const int bx = int(blockIdx.x % unsigned(F.nbx)), j = int(blockIdx.x / unsigned(F.nbx)), lane = threadIdx.x, warp = threadIdx.y;
+  const int row = int(threadIdx.y) / W, warp = int(threadIdx.y) % W, lane = threadIdx.x;
+  const int bx = int(blockIdx.x % unsigned(F.nbx)), j = int(blockIdx.x / unsigned(F.nbx)) * R + row;
   const int nx = g.nx, ny = g.ny, nz = g.nz, i = bx * 32 + lane;
-  const bool in = i < nx;
+  const bool in = i < nx && j < ny;
   const float* const* V = F.V[par];
   auto L = [&](int ch, int a, int b, int c) { return __ldg(V[ch] + g.at(clampi(a, 0, nx), clampi(b, 0, ny), clampi(c, 0, nz))); };
   auto cvel = [&](int a, int b, int c, float v[3]) {
@@ -1321,9 +1331,9 @@ __global__ void __launch_bounds__(32 * kMapWarps) k_maps(Grid g, Uni U, Fields F
   const float dz = U.dzv.x;
   float comp = -30.f, wmx = 0.f, uh = 0.f;
   const int k12 = min(int(12000.f / dz), nz - 1);
-  for (int k0 = 0; k0 < k12; k0 += kMapLevels) {
-    const int n = min(kMapLevels, k12 - k0);
-    for (int t = warp; t < n; t += kMapWarps) {
+  for (int k0 = 0; k0 < k12; k0 += LV) {
+    const int n = min(LV, k12 - k0);
+    for (int t = warp; t < n; t += W) {
       const int k = k0 + t;
       float term = 0.f;
       if (in) {
@@ -1333,20 +1343,20 @@ __global__ void __launch_bounds__(32 * kMapWarps) k_maps(Grid g, Uni U, Fields F
         const float z = (float(k) + 0.5f) * dz;
         if (z > 2000.f && z < 5000.f && w > 0.f) term = w * fmaxf(zeta(k), 0.f) * dz;
       }
-      s_uh[t][lane] = term;
+      s_uh[row][t][lane] = term;
     }
     __syncthreads();
     if (warp == 0)
-      for (int t = 0; t < n; t++) uh += s_uh[t][lane];
+      for (int t = 0; t < n; t++) uh += s_uh[row][t][lane];
     __syncthreads();
   }
-  s_max[0][warp][lane] = comp;
-  s_max[1][warp][lane] = wmx;
+  s_max[0][threadIdx.y][lane] = comp;
+  s_max[1][threadIdx.y][lane] = wmx;
   // radiance of the column from the top down: opacity and temperature of each level, then the sum in order
   float tr = 1.f, bt = 0.f;
-  for (int k0 = nz - 1; k0 >= 0; k0 -= kMapLevels) {
-    const int n = min(kMapLevels, k0 + 1);
-    for (int t = warp; t < n; t += kMapWarps) {
+  for (int k0 = nz - 1; k0 >= 0; k0 -= LV) {
+    const int n = min(LV, k0 + 1);
+    for (int t = warp; t < n; t += W) {
       const int k = k0 - t;
       float a = 0.f, T = 0.f;
       if (in) T = __ldg(V[3] + g.at(i, j, k));
@@ -1356,14 +1366,14 @@ __global__ void __launch_bounds__(32 * kMapWarps) k_maps(Grid g, Uni U, Fields F
                             1.f * __ldg(F.Q[0][3] + o)) * bsA(F.B, nz, k).z * dz;
         a = 1.f - expf(-dtau);
       }
-      s_a[t][lane] = a;
-      s_t[t][lane] = T;
+      s_a[row][t][lane] = a;
+      s_t[row][t][lane] = T;
     }
     __syncthreads();
     if (warp == 0 && tr >= 1e-3f)
       for (int t = 0; t < n; t++) {
-        const float a = s_a[t][lane];
-        bt += tr * a * s_t[t][lane] * bsB(F.B, nz, k0 - t).x;
+        const float a = s_a[row][t][lane];
+        bt += tr * a * s_t[row][t][lane] * bsB(F.B, nz, k0 - t).x;
         tr *= 1.f - a;
         if (tr < 1e-3f) break;
       }
@@ -1371,9 +1381,9 @@ __global__ void __launch_bounds__(32 * kMapWarps) k_maps(Grid g, Uni U, Fields F
   }
   if (warp != 0 || !in) return;
 #pragma unroll
-  for (int w = 1; w < kMapWarps; w++) {
-    comp = fmaxf(comp, s_max[0][w][lane]);
-    wmx = fmaxf(wmx, s_max[1][w][lane]);
+  for (int w = 1; w < W; w++) {
+    comp = fmaxf(comp, s_max[0][row * W + w][lane]);
+    wmx = fmaxf(wmx, s_max[1][row * W + w][lane]);
   }
   const int k1 = clampi(int(1000.f / dz), 1, nz - 2);
   float v0[3], v1[3];
@@ -1791,7 +1801,16 @@ void launch_rain(const Grid& g, const Uni& U, const Fields& F, cudaStream_t s) {
   k_rain<<<grid3(g.nx, g.ny, 1, kB2), kB2, 0, s>>>(g, U, F);
 }
 void launch_maps(const Grid& g, const Uni& U, const Fields& F, int par, float4* out, cudaStream_t s) {
-  k_maps<<<unsigned(F.nbx) * unsigned(g.ny), dim3(32, kMapWarps), 0, s>>>(g, U, facing(F, par), out);
+  // the more columns, the fewer warps to each: 8, 4 and 2 cross where the row blocks of 32 columns number about a thousand
+  // (203 x 157: 1099) and 2600 (260 x 260: 2340, 320 x 320: 3200), above which 2 is never more than a tenth off the best
+  const unsigned rows = unsigned(F.nbx) * unsigned(g.ny);
+  const auto launch = [&](auto k, int w) {
+    const int r = kMapWarps / w;
+    k<<<unsigned(F.nbx) * unsigned((g.ny + r - 1) / r), dim3(32, kMapWarps), 0, s>>>(g, U, facing(F, par), out);
+  };
+  if (rows <= 1024) launch(k_maps<8>, 8);
+  else if (rows <= 2600) launch(k_maps<4>, 4);
+  else launch(k_maps<2>, 2);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
