@@ -1801,15 +1801,14 @@ void launch_rain(const Grid& g, const Uni& U, const Fields& F, cudaStream_t s) {
   k_rain<<<grid3(g.nx, g.ny, 1, kB2), kB2, 0, s>>>(g, U, F);
 }
 void launch_maps(const Grid& g, const Uni& U, const Fields& F, int par, float4* out, cudaStream_t s) {
-  // the more columns, the fewer warps to each: 8, 4 and 2 cross where the row blocks of 32 columns number about a thousand
-  // (203 x 157: 1099) and 2600 (260 x 260: 2340, 320 x 320: 3200), above which 2 is never more than a tenth off the best
+  // two from where the row blocks of 32 columns number 2560 (260 x 260: 2340, 320 x 320: 3200). Four would gain 2 us at 203 x
+  // 157 and 260 x 260 with the fields in L2, but lose 4 at 256 x 224 x 40 without (47 -> 51 us)
   const unsigned rows = unsigned(F.nbx) * unsigned(g.ny);
   const auto launch = [&](auto k, int w) {
     const int r = kMapWarps / w;
     k<<<unsigned(F.nbx) * unsigned((g.ny + r - 1) / r), dim3(32, kMapWarps), 0, s>>>(g, U, facing(F, par), out);
   };
-  if (rows <= 1024) launch(k_maps<8>, 8);
-  else if (rows <= 2600) launch(k_maps<4>, 4);
+  if (rows <= 2560) launch(k_maps<8>, 8);
   else launch(k_maps<2>, 2);
 }
 

@@ -14,8 +14,8 @@ def _model(nx, ny, nz, scheme):
     return M.setup_case(W.StormCase("maps", nx, ny, nz, 1000.0, 6.0, 1, scheme=scheme, bubbles=[], noise=0.0))[0]
 
 
-# row blocks of 32 columns: 1024 (eight warps to a column), 1025, 1402 (four, rows left over), 2600, 2601, 3003 (two)
-@pytest.mark.parametrize("nx,ny,nz,scheme", [(20, 1024, 16, 0), (20, 1025, 16, 1), (61, 701, 40, 0), (33, 1300, 28, 1), (17, 2601, 16, 0),
+# row blocks of 32 columns: 2560 (eight warps to a column), 2561 and more (two; rows left over in the last block)
+@pytest.mark.parametrize("nx,ny,nz,scheme", [(20, 2560, 16, 0), (20, 2561, 16, 1), (61, 1402, 40, 0), (33, 1300, 28, 1), (17, 2603, 16, 0),
                                              (90, 1001, 9, 1), (64, 1501, 100, 0)])
 def test_same_columns_same_maps(native, nx, ny, nz, scheme):
     r = np.random.default_rng(nx + ny)
