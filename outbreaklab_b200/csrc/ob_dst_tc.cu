@@ -342,7 +342,7 @@ __device__ __forceinline__ void dst_tc_run(const Src& src, unsigned int* err) {
       const TcOut& out = ti.out;
       const int BN = ti.BN, m0 = ti.m0, n0 = ti.n0;
       const int b = it & 1;
-      if (!tc::mbar_wait(&tfull[b], (it >> 1) & 1, err, 8u)) break;
+      if (!tc::mbar_wait_warp(&tfull[b], (it >> 1) & 1, err, 8u)) break;
       tc::tc_fence_after();
       const int m = m0 + q * 32 + lane;  // this thread's row of the tile
       const bool mv = m < out.M;
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         prefetch_rows(out, mtn * 2 * BM + int(rank) * BM + q * 32 + lane, n0n, cen - n0n);
       }
       const int b = it & 1;
-      if (!tc::mbar_wait(&tfull[b], (it >> 1) & 1, err, 8u)) break;
+      if (!tc::mbar_wait_warp(&tfull[b], (it >> 1) & 1, err, 8u)) break;
       tc::tc_fence_after();
       const int m = m0 + q * 32 + lane;
       const bool mv = m < out.M;

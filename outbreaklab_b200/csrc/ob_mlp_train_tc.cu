@@ -229,10 +229,10 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_mlp_step(const __grid_const
     __syncthreads();
     if (ctl) {
       if (lane == 0) {
-        if (ph == 0) tc::mbar_wait(wbar, 0, err, 1u);
+        if (ph == 0) ok = tc::mbar_wait(wbar, 0, err, 1u);   // without weights no product is begun
         tc::tc_fence_after();
         const uint32_t sw = tc::smem_u32(sm);
-        switch (ph) {   // the first layer has 12 inputs, dY 10 outputs: one step of K (the rest of their images is zero)
+        if (ok) switch (ph) {   // the first layer has 12 inputs, dY 10 outputs: one step of K (the rest of their images is zero)
           case 0: issue_layer(tmem, sa, sw + S_W1, NH, 16, NH, bar); break;
           case 1: issue_layer(tmem + NH, sa, sw + S_W2, NH, NH, NH, bar); break;
           case 2: issue_layer(tmem + 2 * NH, sa, sw + S_W3, NH, NH, NH, bar); break;
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_mlp_step(const __grid_const
       __syncwarp();
       continue;
     }
-    if (ok) ok = tc::mbar_wait(bar, uint32_t(ph & 1), err, 4u);
+    if (ok) ok = tc::mbar_wait_warp(bar, uint32_t(ph & 1), err, 4u);
     tc::tc_fence_after();
     if (ph < 3) {   // hidden layer: bias, GELU; its derivative takes Z's place in TMEM for the way back
       const float* bias = P.w + (ph == 0 ? OB1 : ph == 1 ? OB2 : OB3) + c0;
@@ -293,7 +293,9 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) k_mlp_step(const __grid_const
       if (ok) put_features(l > 0 ? act : nullptr, P.dZt[l], P.B, row, c0, s, lane, v);
     }
   }
-  // every product is complete once the sample threads have waited for the last one
+  // every product is complete once the sample threads have waited for the last one; where a wait ran out, what is in flight gets
+  // that long again before its memory is given up
+  if (ctl && lane == 0) tc::mbar_wait(ok ? bar : wbar, 0, err, ok ? 4u : 1u);
   tc::tc_fence_before();
   __syncthreads();
   if (ctl) {
@@ -359,7 +361,7 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_mlp_wgrad(const __grid_constant
     tc::mma_commit(accf);
   }
   if (warp >= 2) {
-    ok = tc::mbar_wait(accf, 0, err, 4u);
+    ok = tc::mbar_wait_warp(accf, 0, err, 4u);
     tc::tc_fence_after();
     const int q = warp & 3, row = q * 32 + lane;
     const uint32_t trow = tmem + (uint32_t(q * 32) << 16);

@@ -42,6 +42,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
   if (err) atomicOr(err, code);
   return false;
 }
+// the same by every lane of a warp that goes on to work as one (shuffles, warp barriers, TMEM loads): the tries of its lanes
+// may run out at different moments, and a lane left alone with such an instruction would wait without a limit
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned int* err, unsigned int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code));
+}
 
 // Programmatic dependent launch: a kernel launched with that attribute may start while the kernel before it in the stream
 // still runs. grid_wait returns once that kernel has completed and its writes are visible (at once when there is none);
