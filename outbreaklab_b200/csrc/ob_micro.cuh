@@ -133,7 +133,6 @@ __device__ __forceinline__ void micro_processes(const Uni& U, float dt, float p0
   m.T = T; m.qv = qv; m.qc = qc; m.qi = qi; m.qr = qr; m.qs = qs; m.qg = qg; m.nr = nr;
 }
 
-// the 3-iteration mixed-phase saturation adjustment that closes the block (model.js:893-905)
 // Vapour that a bound from below on the saturation value already exceeds: the adjustment of a cloudless cell then finds
 // nothing to condense and nothing to evaporate and changes nothing. One approximate exponential and quotient stand for the
 // two exponentials, the divisions and the branches of the full form. The bound: mix(esl, esi, f) is at least the smaller of
@@ -145,10 +144,10 @@ __device__ __forceinline__ bool far_below_saturation(float T, float p0, float qv
   const float x = (ice ? 21.8745584f : 17.67f) * __fdividef(T - (ice ? 273.16f : T0K), T - (ice ? 7.66f : 29.65f));
   return p0 >= 100.f && T > 100.f && qv * p0 < 0.99f * 0.622f * 611.2f * __expf(x);
 }
+// the 3-iteration mixed-phase saturation adjustment that closes the block (model.js:893-905)
 __device__ __forceinline__ void sat_adjust(float p0, MCell& m) {
   if (m.qc == 0.f && m.qi == 0.f && far_below_saturation(m.T, p0, m.qv)) return;
   float T = m.T, qv = m.qv, qc = m.qc, qi = m.qi;
-  // mixed-phase saturation adjustment, 3 iterations (model.js:893-905)
   const float qi0 = qi;
   float qcl = qc + qi, dsum = 0.f;
   for (int it = 0; it < 3; it++) {

@@ -171,7 +171,10 @@ __device__ __forceinline__ bool low_mode(int l, int m) { return l < 2 && m < 2; 
 // recurrence, whose two IEEE divisions per level are the rest of the time. The lowest 2 x 2 modes run in FP64 in their
 // own threads of the same launch, their columns in cpd. 464 x 464 x 60: 61 us against 69 us for a kernel that kept c' and
 // the column in global memory plus 47 us for the lowest modes in a launch of their own.
-constexpr int kTriThreads = 64, kTriBatch = 16, kTriSmemLevels = 440;   // 440 levels: 220 KB
+// 440 levels (220 KB) is what shared memory holds; there one block of two warps is all an SM has, and whether that still
+// pays depends on the grid: whole solves at 440 levels against 441, which take k_tri_f32_any, 289 and 521 us at 64 x 64, 441 and
+// 765 at 128 x 128, 1.86 and 1.97 ms at 240 x 240, but 9.7 and 8.3 at 464 x 464.
+constexpr int kTriThreads = 64, kTriBatch = 16, kTriSmemLevels = 440;
 __global__ void __launch_bounds__(kTriThreads) k_tri_f32(int nx, int ny, int nz, const float* __restrict__ lam,
                                                          const float4* __restrict__ zop, float* __restrict__ hat,
                                                          double* __restrict__ cpd) {

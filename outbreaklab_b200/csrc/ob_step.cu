@@ -840,9 +840,9 @@ __device__ __forceinline__ unsigned warp_append(unsigned* ctr) {
 // one texel of the physics pass; returns the hydrometeor and spare channels that the cell's new state holds (bits 1..7). MM: microphysics as the
 // scheme (kMicroPlain), the scheme plus sampled (state, tendency) pairs (kMicroRecord), or queued for the surrogate
 // kernel where it can act (kMicroSurrogate).
-// Neighbour reads clamp to the edge of their texture (textureLoad with clamped coordinates, model.js:596-606): the
-// offsets below are the clamped index minus the texel's own, for the staggered box [0, n] (V) and the cell box
-// [0, n-1] (Q, aux, phi_t), computed once per texel. BND: boundary air masses present (else the target state is the
+// Neighbour reads clamp to the edge of their texture (textureLoad with clamped coordinates, model.js:596-606): the byte
+// offsets below are those of the clamped neighbours, for the staggered box [0, n] (V) and the cell box [0, n-1] (Q, aux,
+// phi_t), computed once per texel. BND: boundary air masses present (else the target state is the
 // base state, see tgtUb).
 template <bool BND, int MM, bool HUR = false>
 __device__ __forceinline__ unsigned phys_texel(const Grid& g, const Uni& U, const Fields& F, int par, int ci, int cj, int ck, bool dry,
